@@ -82,6 +82,127 @@ hsdr_decode_rows_kernel(const float* __restrict__ D, const uint16_t* __restrict_
     }
 }
 
+// The whole matrix at once. A CTA keeps one slice of every atom (4 * LANES consecutive elements,
+// [K][4 * LANES] floats) in shared memory and walks tiles; LANES lanes rebuild a tile's slice, four
+// elements each, so an atom row is one conflict-free 128-bit read per lane. hsdr_decode_rows_kernel
+// re-reads every atom from L2 for every tile instead: 1.6 GB for 4099 x 4101 in 128 x 128 tiles,
+// scalar where the width is odd (365 us); here the same bytes come from shared memory, whose
+// bandwidth (about 45 us of it) and the issue of ten instructions a code are the bound: 75 us, and
+// 65 us where the width is a multiple of four. 32 warps on an SM hide the reads of codes and atoms
+// (16: 86 us). The (slice, tile) pairs are dealt to the CTAs, one an SM, in equal contiguous runs,
+// so a CTA stages one to three slices. Sums as above: stage-major, slot-minor, one multiplication and
+// one addition per code, never contracted.
+constexpr uint32_t kTilesThreads = 1024;
+
+__device__ __forceinline__ unsigned long long mul2_rn(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long add2_rn(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// QUAD: k is a multiple of four and the stream 8-byte aligned, so four codes are one read.
+template <int LANES, bool QUAD>
+__global__ void __launch_bounds__(kTilesThreads, 1)
+hsdr_decode_tiles_kernel(const float* __restrict__ D, const uint16_t* __restrict__ codes, const float* __restrict__ scales,
+                         const float* __restrict__ edges, DecodeGeom g, uint32_t n_tiles, uint32_t n_slices, uint32_t vec_out,
+                         float* __restrict__ out) {
+    extern __shared__ __align__(16) float atoms_s[];            // [K][4 * LANES]
+    constexpr uint32_t W = 4u * LANES, kGroups = kTilesThreads / LANES;
+    const uint32_t tid = threadIdx.x, lane = tid % LANES, grp = tid / LANES;
+    const uint32_t T = g.Tr * g.Tc, slots = g.S * g.k;
+    const uint64_t units = static_cast<uint64_t>(n_slices) * n_tiles;
+    const uint64_t lo = units * blockIdx.x / gridDim.x, hi = units * (blockIdx.x + 1u) / gridDim.x;
+    const uint32_t step_br = kGroups / g.n_ct, step_bc = kGroups % g.n_ct;
+    for (uint64_t u = lo; u < hi;) {
+        const uint32_t slice = static_cast<uint32_t>(u / n_tiles), t_lo = static_cast<uint32_t>(u - static_cast<uint64_t>(slice) * n_tiles);
+        const uint32_t t_hi = static_cast<uint32_t>(min(static_cast<uint64_t>(n_tiles), t_lo + (hi - u)));
+        u += t_hi - t_lo;
+        const uint32_t p0 = slice * W;
+        __syncthreads();                                        // the previous slice is no longer read
+        if ((T & 3u) == 0u) {
+            const uint32_t w4 = min(W, T - p0) / 4u;
+            for (uint32_t i = tid; i < g.K * LANES; i += kTilesThreads) {
+                const uint32_t a = i / LANES, c = i % LANES;
+                if (c < w4)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                     static_cast<uint32_t>(__cvta_generic_to_shared(atoms_s + a * W + c * 4u))),
+                                 "l"(D + static_cast<size_t>(a) * T + p0 + c * 4u)
+                                 : "memory");
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        } else {
+            const uint32_t w1 = min(W, T - p0);
+            for (uint32_t i = tid; i < g.K * W; i += kTilesThreads) {
+                const uint32_t a = i / W, c = i % W;
+                if (c < w1) atoms_s[i] = __ldg(D + static_cast<size_t>(a) * T + p0 + c);
+            }
+        }
+        // where this lane's four elements go inside a tile's place in the matrix
+        const uint32_t p = p0 + lane * 4u;
+        uint32_t off[4];
+#pragma unroll
+        for (uint32_t e = 0; e < 4u; ++e) off[e] = (p + e) / g.Tc * g.C + (p + e) % g.Tc;
+        const uint32_t n_el = p < T ? min(4u, T - p) : 0u;
+        __syncthreads();
+        const float* mine = atoms_s + lane * 4u;
+        uint32_t tile = t_lo + grp, br = tile / g.n_ct, bc = tile - br * g.n_ct;
+        for (; tile < t_hi; tile += kGroups) {
+            const uint16_t* tc = codes + static_cast<size_t>(tile) * slots;
+            unsigned long long v0 = 0ull, v1 = 0ull;
+            auto add = [&](uint32_t code, uint32_t gbits) {
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(mine + (code & 0x7FFFu) * W);
+                const uint32_t sb = gbits ^ ((code & 0x8000u) << 16);
+                const unsigned long long s2 = (static_cast<unsigned long long>(sb) << 32) | sb;
+                v0 = add2_rn(v0, mul2_rn(s2, a.x));
+                v1 = add2_rn(v1, mul2_rn(s2, a.y));
+            };
+            for (uint32_t l = 0; l < g.S; ++l) {
+                const uint32_t gbits = __float_as_uint(__ldg(scales + l));
+                if constexpr (QUAD) {
+#pragma unroll 2
+                    for (uint32_t kk = 0; kk < g.k; kk += 4u) {
+                        const uint2 c = __ldg(reinterpret_cast<const uint2*>(tc + l * g.k + kk));
+                        add(c.x & 0xFFFFu, gbits);
+                        add(c.x >> 16, gbits);
+                        add(c.y & 0xFFFFu, gbits);
+                        add(c.y >> 16, gbits);
+                    }
+                } else {
+#pragma unroll 4
+                    for (uint32_t kk = 0; kk < g.k; ++kk) add(__ldg(tc + l * g.k + kk), gbits);
+                }
+            }
+            float* dst = out + static_cast<size_t>(br) * g.Tr * g.C + static_cast<size_t>(bc) * g.Tc;
+            if (vec_out && n_el == 4u) {
+                *reinterpret_cast<ulonglong2*>(dst + off[0]) = make_ulonglong2(v0, v1);
+            } else {
+                if (n_el > 0u) dst[off[0]] = __uint_as_float(static_cast<uint32_t>(v0));
+                if (n_el > 1u) dst[off[1]] = __uint_as_float(static_cast<uint32_t>(v0 >> 32));
+                if (n_el > 2u) dst[off[2]] = __uint_as_float(static_cast<uint32_t>(v1));
+                if (n_el > 3u) dst[off[3]] = __uint_as_float(static_cast<uint32_t>(v1 >> 32));
+            }
+            br += step_br;
+            bc += step_bc;
+            if (bc >= g.n_ct) {
+                bc -= g.n_ct;
+                ++br;
+            }
+        }
+    }
+    // raw strips: top-right, then bottom
+    const uint32_t we = g.C - g.Cf;
+    const uint64_t n_top = static_cast<uint64_t>(g.Rf) * we, n_edge = n_top + static_cast<uint64_t>(g.R - g.Rf) * g.C;
+    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(kTilesThreads) + tid; i < n_edge; i += static_cast<uint64_t>(gridDim.x) * kTilesThreads) {
+        if (i < n_top) out[i / we * g.C + g.Cf + i % we] = edges[i];
+        else out[static_cast<uint64_t>(g.Rf) * g.C + (i - n_top)] = edges[i];
+    }
+}
+
 enum Fmt { F32 = 0, F16, BF16, I8, Q4_0, Q8_0, Q4_K, Q5_K, Q6_K };
 
 __global__ void dequant_simple_kernel(int fmt, const uint8_t* __restrict__ p, size_t n_out,
@@ -240,6 +361,28 @@ void launch_decode_rows(csdr_context* ctx, const csdr_segment* seg, const int32_
     DecodeGeom dg{g.rows, g.cols, g.rows_full, g.cols_full, g.tile_rows, g.tile_cols,
                   g.n_col_tiles, g.n_stages, g.k, g.n_atoms};
     const float* edges = seg->edges ? static_cast<const float*>(seg->edges->ptr) : nullptr;
+    // Whole matrices whose codes read the dictionary often enough to pay for staging it (twice over),
+    // and whose atoms' slices fit shared memory: 64 elements of each up to 880 atoms, 32 up to 1760.
+    const uint64_t T = g.tile_dim();
+    const size_t smem64 = static_cast<size_t>(g.n_atoms) * 256u;
+    if (!rows_dev && n_rows == g.rows && g.n_tiles && T >= 32u && T <= 0x7FFFFFFFull && smem64 / 2u <= ctx->smem_optin &&
+        static_cast<uint64_t>(g.n_tiles) * g.slots() >= 2ull * g.n_atoms) {
+        const bool wide = smem64 <= ctx->smem_optin;
+        const size_t smem = wide ? smem64 : smem64 / 2u;
+        const uint32_t w = wide ? 64u : 32u;
+        const bool quad = g.k % 4u == 0 && (reinterpret_cast<uintptr_t>(seg->codes_ptr()) & 7u) == 0;
+        auto kern = wide ? (quad ? hsdr_decode_tiles_kernel<16, true> : hsdr_decode_tiles_kernel<16, false>)
+                         : (quad ? hsdr_decode_tiles_kernel<8, true> : hsdr_decode_tiles_kernel<8, false>);
+        ctx->opt_in_smem(reinterpret_cast<const void*>(kern), smem);
+        const uint32_t n_slices = static_cast<uint32_t>((T + w - 1u) / w);
+        const uint32_t vec_out = g.cols % 4u == 0 && g.tile_cols % 4u == 0 && (reinterpret_cast<uintptr_t>(out_dev) & 15u) == 0;
+        LaunchScope ls(ctx, KC_DECODE_ROWS);
+        kern<<<static_cast<uint32_t>(ctx->sm_count), kTilesThreads, smem, ctx->stream>>>(
+            static_cast<const float*>(seg->atoms->ptr), seg->codes_ptr(), static_cast<const float*>(seg->scales->ptr), edges, dg,
+            g.n_tiles, n_slices, vec_out, out_dev);
+        ls.done("hsdr_decode_tiles_kernel");
+        return;
+    }
     const bool vec = (g.cols % 4u == 0) && (g.tile_cols % 4u == 0);
     const uint32_t per_block = 256u * (vec ? 4u : 1u);
     dim3 grid(static_cast<unsigned>(n_rows), (g.cols + per_block - 1u) / per_block, 1);
