@@ -256,7 +256,7 @@ void linear(csdr_decoder* d, const Linear& l, const float* x, uint32_t T, float*
         a.batch = T;
         a.y = y;
         a.y_layout = CSDR_LAYOUT_TOKEN_MAJOR;
-        launch_dense_matmul(d->ctx, F(l.raw), l.rows_local, l.cols, a);
+        launch_dense_matmul(d->ctx, F(l.raw), l.rows_local, l.cols, a, false);
     } else {
         rethrow_last(csdr_matmul_device_async(d->ctx, l.use(), x, CSDR_DTYPE_F32, CSDR_LAYOUT_TOKEN_MAJOR, T, y,
                                               CSDR_LAYOUT_TOKEN_MAJOR, nullptr));

@@ -331,7 +331,7 @@ int csdr_archive_matmul_for_layer(csdr_archive* ar, const char* name, const floa
         a.x = buf;
         a.batch = batch;
         a.y = reinterpret_cast<float*>(buf + xoff);
-        launch_dense_matmul(ctx, static_cast<const float*>(it->second->ptr), R, C, a);
+        launch_dense_matmul(ctx, static_cast<const float*>(it->second->ptr), R, C, a, false);
         CSDR_CUDA(cudaMemcpyAsync(y, buf + xoff, yb, cudaMemcpyDeviceToHost, ctx->stream));
         CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
     });

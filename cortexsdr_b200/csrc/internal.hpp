@@ -131,6 +131,7 @@ struct csdr_context {
     bool pdl = true;         // CSDR_PDL=0 launches without programmatic dependent launch
     bool tensor_cores = true;   // CSDR_TENSOR_CORES=0 keeps wide batches on the CUDA-core kernels
     bool tma = true;            // CSDR_TMA=0 keeps the register-fed tensor-core kernel
+    size_t simt_min_batch = 5;  // CSDR_SIMT_MIN_BATCH: smallest batch of row tiles sent to the fp32 projection instead of the one-launch GEMV
     size_t tc_min_batch = 8;    // CSDR_TC_MIN_BATCH: smallest batch sent to the tcgen05 path
     // Per-device launch facts, remembered per context (function attributes and occupancy belong
     // to a device; a process may hold contexts on several).
@@ -222,7 +223,12 @@ size_t dequant_output_count(int fmt_id, size_t nbytes);  // throws on bad size
 void launch_gather_tile(csdr_context* ctx, const csdr_segment* seg, const float* dx, int mt, float* y, int y_layout,
                         uint32_t m_total, uint32_t b0, uint32_t m, const float* bias);
 
+// y = W x (+ bias), fp32. w_fresh: W was written by earlier work on the stream.
 void launch_dense_matmul(csdr_context* ctx, const float* W_dev, uint32_t R, uint32_t C,
-                         const MatmulArgs& a);
+                         const MatmulArgs& a, bool w_fresh);
+
+// Row tiles the tensor-core path refuses (fp32 projection on the CUDA cores, then the gathers).
+bool simt_rows_supported(const csdr_context* ctx, const csdr_segment* seg, size_t batch);
+void matmul_rows_simt(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs& a);
 
 }  // namespace csdr

@@ -25,6 +25,7 @@
 #include <cstdlib>
 
 #include "../internal.hpp"
+#include "gemm_simt.hpp"
 #include "gemm_tcgen05.hpp"
 #include "views.cuh"
 
@@ -1183,6 +1184,39 @@ void launch_matmul_tcgen05(csdr_context* ctx, const csdr_segment* seg, const Mat
     }
     YView yv{a.y, a.y_layout, g.rows, M, 0u, M, a.bias};
     launch_gather_wide(ctx, seg, dx, M, yv, nullptr, TokenScale{});
+}
+
+// One-launch GEMVs take four tokens at a time and 128-bit rows; beyond that, and for widths that
+// are no multiple of four at any batch, Dx comes from the fp32 product and the gathers above read
+// it. The bounds are the gathers' shared memory.
+bool simt_rows_supported(const csdr_context* ctx, const csdr_segment* seg, size_t batch) {
+    const Geometry& g = seg->g;
+    if (!g.row_tiles() || batch > 0xFFFFFFFFull || g.slots() > kWideMaxSlots || g.n_stages > 64u) return false;
+    if (g.cols % 4u == 0 && batch < ctx->simt_min_batch) return false;
+    if (batch > 16u) return gather_wide_smem(g.n_atoms) <= ctx->smem_optin;
+    const size_t rows_per_cta = std::max<size_t>(kGroupThreads, (g.rows + 2u * ctx->sm_count - 1u) / (2u * ctx->sm_count));
+    return rows_per_cta * g.slots() * 2u + static_cast<size_t>(g.n_atoms) * 64u + 1024u <= ctx->smem_optin;
+}
+
+void matmul_rows_simt(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs& a) {
+    const Geometry& g = seg->g;
+    const uint32_t M = static_cast<uint32_t>(a.batch);
+    uint32_t mt = M;
+    if (M <= 16u)
+        for (mt = 1; mt < M;) mt <<= 1;
+    float* dx = static_cast<float*>(ctx->scratch_get(0, static_cast<size_t>(g.n_atoms) * std::max(mt, 16u) * 4u));
+    launch_gemm_simt(ctx, static_cast<const float*>(seg->atoms->ptr), g.n_atoms, g.cols, XView{a.x, a.x_dtype, a.x_layout, g.cols, M, 0u, M},
+                     YView{dx, CSDR_LAYOUT_FEATURE_MAJOR, g.n_atoms, mt, 0u, M, nullptr}, false);
+    if (M <= 16u) {
+        WideDx w{};
+        w.base = w.dx[0] = dx;
+        w.floats = static_cast<size_t>(g.n_atoms) * mt;
+        w.stride = w.tile_mt = mt;
+        const WideOut out{a.y, a.bias, nullptr};
+        gather_tile_group(ctx, &seg, 1, w, M, &out, a.y_layout, TokenScale{});
+        return;
+    }
+    launch_gather_wide(ctx, seg, dx, M, YView{a.y, a.y_layout, g.rows, M, 0u, M, a.bias}, nullptr, TokenScale{});
 }
 
 }  // namespace csdr

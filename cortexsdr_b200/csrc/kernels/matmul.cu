@@ -20,6 +20,7 @@
 #include "gemm_tcgen05.hpp"
 #include "gemv_fused.hpp"
 #include "gemv_queue.hpp"
+#include "gemm_simt.hpp"
 #include "views.cuh"
 
 namespace cg = cooperative_groups;
@@ -461,34 +462,6 @@ hsdr_edge_kernel(const float* __restrict__ edges, uint32_t R, uint32_t C, uint32
     }
 }
 
-// ---------------------------------------------------------------------------
-// Dense rows: y[r][b] = sum_c W[r][c] * x[c][b]. One warp per row.
-// ---------------------------------------------------------------------------
-template <int MT>
-__global__ void __launch_bounds__(256)
-dense_rows_kernel(const float* __restrict__ W, uint32_t R, uint32_t C, XView xv, YView yv) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t r = blockIdx.x * 8u + (threadIdx.x >> 5);
-    if (r >= R) return;
-    const float* w = W + static_cast<size_t>(r) * C;
-    float acc[MT];
-#pragma unroll
-    for (int b = 0; b < MT; ++b) acc[b] = 0.0f;
-    for (uint32_t c = lane; c < C; c += 32u) {
-        const float wv = w[c];
-#pragma unroll
-        for (int b = 0; b < MT; ++b)
-            if (b < xv.M) acc[b] = fmaf(wv, load_x(xv, c, b), acc[b]);
-    }
-#pragma unroll
-    for (int b = 0; b < MT; ++b) {
-        float v = acc[b];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
-        if (lane == 0 && b < yv.M) yv.y[y_index(yv, r, b)] = v + (yv.bias ? yv.bias[r] : 0.0f);
-    }
-}
-
 // y (token-major or feature-major, + bias) from a feature-major product t[r][stride].
 __global__ void __launch_bounds__(256)
 retile_bias_kernel(const float* __restrict__ t, uint32_t R, uint32_t M, uint32_t stride, YView yv) {
@@ -700,17 +673,10 @@ void launch_unpack(csdr_context* ctx, const uint16_t* codes, size_t n, int32_t* 
 }
 
 void launch_dense_matmul(csdr_context* ctx, const float* W, uint32_t R, uint32_t C,
-                         const MatmulArgs& a) {
-    for (size_t b0 = 0; b0 < a.batch; b0 += 16) {
-        const uint32_t m = static_cast<uint32_t>(std::min<size_t>(16, a.batch - b0));
-        XView xv{a.x, a.x_dtype, a.x_layout, C, static_cast<uint32_t>(a.batch), static_cast<uint32_t>(b0), m};
-        YView yv{a.y, a.y_layout, R, static_cast<uint32_t>(a.batch), static_cast<uint32_t>(b0), m, a.bias};
-        dispatch_mt(pick_mt(m), [&](auto mt) {
-            LaunchScope ls(ctx, KC_DENSE);
-            dense_rows_kernel<decltype(mt)::value><<<(R + 7u) / 8u, 256, 0, ctx->stream>>>(W, R, C, xv, yv);
-            ls.done("dense_rows_kernel");
-        });
-    }
+                         const MatmulArgs& a, bool w_fresh) {
+    const uint32_t M = static_cast<uint32_t>(a.batch);
+    launch_gemm_simt(ctx, W, R, C, XView{a.x, a.x_dtype, a.x_layout, C, M, 0u, M}, YView{a.y, a.y_layout, R, M, 0u, M, a.bias},
+                     w_fresh);
 }
 
 void launch_matmul(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs& a) {
@@ -729,8 +695,9 @@ void launch_matmul(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs&
             return;
         }
     }
-    if (!g.row_tiles() && ctx->cache_2d && ctx->tensor_cores && a.batch >= 16 && g.rows % 128u == 0 && g.cols % 8u == 0 &&
-        g.rows <= 0x7FFFu * 128u) {
+    const bool planes_2d = !g.row_tiles() && ctx->cache_2d && ctx->tensor_cores && g.rows % 128u == 0 && g.cols % 8u == 0 &&
+                           g.rows <= 0x7FFFu * 128u;
+    if (planes_2d && a.batch >= 16) {
         // 2-D tiles at a wide batch: what the reference does (decompress once, keep the layer, dense
         // product - SparseInferenceEngine.cpp:1301-1310 behind its layer cache), on the tensor cores:
         // the weight is rebuilt once by the bit-exact decode kernel, split into bf16 hi/lo planes that
@@ -768,13 +735,40 @@ void launch_matmul(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs&
         }
         return;
     }
-    const size_t budget = std::min<size_t>(ctx->smem_optin, 200u * 1024u);
+    if (simt_rows_supported(ctx, seg, a.batch)) {
+        matmul_rows_simt(ctx, seg, a);
+        return;
+    }
     const bool fast_rows = g.row_tiles() && (g.cols % 4u == 0);
+    const bool factored_tc = !fast_rows && ctx->tile_tc && ctx->tensor_cores && ctx->tma && g.cols == g.cols_full &&
+                             g.tile_cols % 8u == 0 && (static_cast<size_t>(g.n_atoms) * g.tile_rows) % 128u == 0 &&
+                             a.batch * g.n_col_tiles >= ctx->tc_min_batch &&
+                             a.batch * g.n_col_tiles * g.n_atoms * static_cast<size_t>(g.tile_rows) * 4u <= (1ull << 30);
+    // 2-D tiles whose shape the tensor maps do not take (ragged edges, rows not in 128s): the rebuilt
+    // weight stays with the segment as fp32 (4 bytes an element, as the planes above) and the product
+    // is a plain fp32 one. The factored form moves batch * (n_atoms * tile_rows + rows * slots) words
+    // of tile products per column tile where the weight has rows * tile_cols: taken where that is
+    // more, and from 16 tokens on; a weight below a megabyte is bound by launches either way and
+    // keeps the factored form, which needs no copy of it.
+    if (!g.row_tiles() && ctx->cache_2d && !planes_2d &&
+        (a.batch >= 16 ||
+         (a.batch * (static_cast<size_t>(g.n_atoms) * g.tile_rows + static_cast<size_t>(g.rows) * g.slots()) >=
+              static_cast<size_t>(g.rows) * g.tile_cols &&
+          (!factored_tc || static_cast<size_t>(g.rows) * g.cols >= (1u << 18))))) {
+        if (!seg->dense) {
+            auto dn = std::make_shared<csdr_segment>();
+            dn->ctx = ctx;
+            dn->atoms = std::make_shared<DeviceBuffer>(static_cast<size_t>(g.rows) * g.cols * 4u, ctx->device);
+            launch_decode_rows(ctx, seg, nullptr, g.rows, static_cast<float*>(dn->atoms->ptr));
+            CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
+            seg->dense = dn;
+        }
+        launch_dense_matmul(ctx, static_cast<const float*>(seg->dense->atoms->ptr), g.rows, g.cols, a, false);
+        return;
+    }
+    const size_t budget = std::min<size_t>(ctx->smem_optin, 200u * 1024u);
     const bool fast_tiles = !fast_rows && (g.tile_cols % 4u == 0);
-    if (!fast_rows && ctx->tile_tc && ctx->tensor_cores && ctx->tma && g.cols == g.cols_full && g.tile_cols % 8u == 0 &&
-        (static_cast<size_t>(g.n_atoms) * g.tile_rows) % 128u == 0 &&
-        a.batch * g.n_col_tiles >= ctx->tc_min_batch &&
-        a.batch * g.n_col_tiles * g.n_atoms * static_cast<size_t>(g.tile_rows) * 4u <= (1ull << 30)) {
+    if (factored_tc) {
         // 2-D tiles, a few tokens: the tile products are ONE GEMM - the dictionary read as
         // K * Tr rows of Tc columns against the activations read as batch * n_ct tokens of Tc
         // columns (a token-major activation row IS its n_ct column tiles one after the other) -
@@ -826,7 +820,7 @@ void launch_matmul(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs&
         float* W = static_cast<float*>(
             ctx->scratch_get(2, static_cast<size_t>(g.rows) * g.cols * sizeof(float)));
         launch_decode_rows(ctx, seg, nullptr, g.rows, W);
-        launch_dense_matmul(ctx, W, g.rows, g.cols, a);
+        launch_dense_matmul(ctx, W, g.rows, g.cols, a, true);
         return;
     }
     for (size_t b0 = 0; b0 < a.batch; b0 += mt_cap) {
