@@ -1186,13 +1186,17 @@ void launch_matmul_tcgen05(csdr_context* ctx, const csdr_segment* seg, const Mat
     launch_gather_wide(ctx, seg, dx, M, yv, nullptr, TokenScale{});
 }
 
-// One-launch GEMVs take four tokens at a time and 128-bit rows; beyond that, and for widths that
-// are no multiple of four at any batch, Dx comes from the fp32 product and the gathers above read
-// it. The bounds are the gathers' shared memory.
+// Widths that are no multiple of four have no 128-bit rows: Dx comes from the fp32 product at any
+// batch, and the gathers above read it. Others leave the one-launch GEMV from five tokens on where
+// the dictionary is larger than 2^18 elements (512 atoms of 4096 at 5 tokens: 18.4 against 15.0 us,
+// 300 of 1024: 10.4 against 9.3; 128 of 2048, the size of the line: 10.1 against 11.0 at 5 tokens,
+// 10.2 against 9.4 at 7; 300 of 512, below it: 8.0 against 13.8; up to four tokens 512 of 4096: 11.8
+// against 13.6), and past its sixteen tokens always. The bounds are the gathers' shared memory.
 bool simt_rows_supported(const csdr_context* ctx, const csdr_segment* seg, size_t batch) {
     const Geometry& g = seg->g;
     if (!g.row_tiles() || batch > 0xFFFFFFFFull || g.slots() > kWideMaxSlots || g.n_stages > 64u) return false;
-    if (g.cols % 4u == 0 && batch < ctx->simt_min_batch) return false;
+    if (g.cols % 4u == 0 && (batch < ctx->simt_min_batch || (batch <= 16u && static_cast<size_t>(g.n_atoms) * g.cols < ctx->simt_min_dict)))
+        return false;
     if (batch > 16u) return gather_wide_smem(g.n_atoms) <= ctx->smem_optin;
     const size_t rows_per_cta = std::max<size_t>(kGroupThreads, (g.rows + 2u * ctx->sm_count - 1u) / (2u * ctx->sm_count));
     return rows_per_cta * g.slots() * 2u + static_cast<size_t>(g.n_atoms) * 64u + 1024u <= ctx->smem_optin;
