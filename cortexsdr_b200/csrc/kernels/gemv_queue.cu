@@ -76,7 +76,7 @@ struct QTask {
     const float* D;           // the dictionary in stage blocks (stage_blocks_kernel), not row-major
     const uint16_t* codes;
     const float* scales;
-    const void* x;            // X_PLAIN: activations (dtype, layout); X_TAGGED: u64 words [M][C]
+    const void* x;            // X_PLAIN: fp32 rows [M][C] on 16-byte boundaries; X_TAGGED: u64 words [M][C]
     float* y;                 // fp32 result, or null when only the tagged copy is wanted
     u64* y_tag;               // tagged copy [M][R] for a later task of the list, or null
     const float* bias;
@@ -88,7 +88,7 @@ struct QTask {
     uint32_t n_units;
     uint32_t dx_off;          // word offset of its Dx slot: [K][MT]
     uint32_t rows_per_cta;
-    uint32_t x_kind, x_dtype, x_layout, y_layout;
+    uint32_t x_kind, y_layout;
     uint32_t M;
     float norm_eps;
     uint32_t epilogue;
@@ -154,10 +154,6 @@ __device__ __forceinline__ u64 ld_tagged(const u64* p) {
 __device__ __forceinline__ void st_tagged(u64* p, float value, uint32_t tag) {
     const u64 w = (static_cast<u64>(tag) << 32) | __float_as_uint(value);
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
-}
-
-__device__ __forceinline__ XView x_view(const QTask& t) {
-    return XView{t.x, static_cast<int>(t.x_dtype), static_cast<int>(t.x_layout), t.C, t.M, 0u, t.M};
 }
 
 // Polls `n` tagged words (word i of this lane at src[i * stride]) in batches of B loads in
@@ -264,28 +260,19 @@ __global__ void __launch_bounds__(kThreads, 1) hsdr_gemv_queue_kernel(const __gr
             float* xs = reinterpret_cast<float*>(qsm + static_cast<size_t>(slot) * p.stage_bytes + kAtomsPerUnit * kSlab * 4u);
             const uint32_t bar = smem_u32(&full_bar[slot]);
             if (t.x_kind == X_PLAIN) {
-                const XView xv = x_view(t);
-                const bool rows_contig = xv.layout == CSDR_LAYOUT_TOKEN_MAJOR || xv.Mtotal == 1;
-                if (xv.dtype == CSDR_DTYPE_F32 && rows_contig &&
-                    ((reinterpret_cast<uintptr_t>(xv.x) | (static_cast<uintptr_t>(xv.C) * 4u)) & 15u) == 0) {
-                    // one bulk copy per token, completing on the stage's barrier like the weights
-                    if (lane == 0)
-                        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(xv.M * cw * 4u)
-                                     : "memory");
-                    __syncwarp();
-                    if (lane < xv.M) {
-                        const float* src = static_cast<const float*>(xv.x) + static_cast<size_t>(lane) * xv.C + c0;
-                        asm volatile(
-                            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                smem_u32(xs + lane * kSlab)),
-                            "l"(src), "r"(cw * 4u), "r"(bar)
-                            : "memory");
-                    }
-                } else {
-                    for (uint32_t i = lane; i < MT * kSlab; i += 32u) {
-                        const uint32_t b = i / kSlab, c = i - b * kSlab;
-                        if (c < cw && b < xv.M) xs[i] = load_x(xv, c0 + c, b);
-                    }
+                // fp32 rows on 16-byte boundaries (stage_activations sees to it): one bulk copy per token,
+                // completing on the stage's barrier like the weights
+                if (lane == 0)
+                    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(t.M * cw * 4u)
+                                 : "memory");
+                __syncwarp();
+                if (lane < t.M) {
+                    const float* src = static_cast<const float*>(t.x) + static_cast<size_t>(lane) * t.C + c0;
+                    asm volatile(
+                        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                            smem_u32(xs + lane * kSlab)),
+                        "l"(src), "r"(cw * 4u), "r"(bar)
+                        : "memory");
                 }
             }   // X_TAGGED: the product warps fetch the slab themselves when they reach the stage
             __syncwarp();
@@ -693,6 +680,78 @@ stage_blocks_kernel(const float* __restrict__ D, uint32_t K, uint32_t C, float* 
     }
 }
 
+// Activations the loader cannot copy in bulk (feature-major with several tokens, bf16, unaligned)
+// become fp32 rows, token after token, in one launch before the list's: the loader warp reading them
+// element by element held the whole ring up (12 products of 5769x4096 at two feature-major tokens:
+// 312 us). grid (chunks, activations).
+struct XRowsJob {
+    const void* x;
+    float* out;
+    uint32_t C, dtype, layout;
+};
+struct XRowsParams {
+    XRowsJob job[kMaxQueueTasks];
+    uint32_t M;
+};
+
+__global__ void __launch_bounds__(256) x_rows_kernel(const __grid_constant__ XRowsParams p) {
+    asm volatile("griddepcontrol.launch_dependents;");   // the list's weights may be requested meanwhile
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const XRowsJob& j = p.job[blockIdx.y];
+    const XView xv{j.x, static_cast<int>(j.dtype), static_cast<int>(j.layout), j.C, p.M, 0u, p.M};
+    for (uint32_t c = blockIdx.x * 256u + threadIdx.x; c < j.C; c += gridDim.x * 256u)
+        for (uint32_t b = 0; b < p.M; ++b) j.out[static_cast<size_t>(b) * j.C + c] = load_x(xv, c, b);
+}
+
+bool bulk_rows(const QueueItem& it) {
+    return it.x_dtype == CSDR_DTYPE_F32 && (it.x_layout == CSDR_LAYOUT_TOKEN_MAJOR || it.batch == 1) &&
+           ((reinterpret_cast<uintptr_t>(it.x) | (static_cast<uintptr_t>(it.seg->g.cols) * 4u)) & 15u) == 0;
+}
+
+// Stages what needs it and points the tasks at the rows. Tasks that read another's result stay.
+void stage_activations(csdr_context* ctx, const QueueItem* items, uint32_t n, QTask* tasks) {
+    XRowsParams xp{};
+    uint32_t n_jobs = 0, job_of[kMaxQueueTasks] = {}, max_c = 0;
+    bool staged[kMaxQueueTasks] = {};
+    size_t floats = 0, at[kMaxQueueTasks] = {};
+    for (uint32_t i = 0; i < n; ++i) {
+        const QueueItem& it = items[i];
+        if (it.dep >= 0 || bulk_rows(it)) continue;
+        staged[i] = true;
+        uint32_t j = 0;
+        for (; j < n_jobs; ++j)
+            if (xp.job[j].x == it.x && xp.job[j].C == it.seg->g.cols && xp.job[j].dtype == static_cast<uint32_t>(it.x_dtype) &&
+                xp.job[j].layout == static_cast<uint32_t>(it.x_layout))
+                break;
+        if (j == n_jobs) {
+            xp.job[j] = XRowsJob{it.x, nullptr, it.seg->g.cols, static_cast<uint32_t>(it.x_dtype), static_cast<uint32_t>(it.x_layout)};
+            at[j] = floats;
+            floats += (static_cast<size_t>(it.batch) * it.seg->g.cols + 3u) & ~static_cast<size_t>(3);
+            max_c = std::max(max_c, it.seg->g.cols);
+            ++n_jobs;
+        }
+        job_of[i] = j;
+    }
+    if (!n_jobs) return;
+    float* rows = static_cast<float*>(ctx->scratch_get(5, floats * 4u));
+    for (uint32_t j = 0; j < n_jobs; ++j) xp.job[j].out = rows + at[j];
+    xp.M = static_cast<uint32_t>(items[0].batch);
+    for (uint32_t i = 0; i < n; ++i)
+        if (staged[i]) tasks[i].x = xp.job[job_of[i]].out;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((max_c + 255u) / 256u, n_jobs, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    LaunchScope ls(ctx, KC_GEMV_QUEUE);
+    CSDR_CUDA(cudaLaunchKernelEx(&cfg, x_rows_kernel, xp));
+    ls.done("x_rows_kernel");
+}
+
 // Built on a dictionary's first use by the list kernel and kept with it (as many bytes again as the
 // atoms): not inside a stream capture, like every first use that allocates.
 const DeviceBuffer* stage_blocks_of(csdr_context* ctx, const csdr_segment* seg) {
@@ -838,8 +897,6 @@ void launch_gemv_queue(csdr_context* ctx, const QueueItem* items, uint32_t n) {
             t.unit0 = unit;
             t.n_units = (g.n_atoms + kAtomsPerUnit - 1u) / kAtomsPerUnit;
             t.rows_per_cta = rows_per_cta_for(ctx, g.rows);
-            t.x_dtype = static_cast<uint32_t>(it.x_dtype);
-            t.x_layout = static_cast<uint32_t>(it.x_layout);
             t.y_layout = static_cast<uint32_t>(it.y_layout);
             t.M = batch;
             t.epilogue = it.swiglu_gate ? EPI_SWIGLU : EPI_PLAIN;
@@ -847,6 +904,7 @@ void launch_gemv_queue(csdr_context* ctx, const QueueItem* items, uint32_t n) {
             max_k = std::max(max_k, g.n_atoms);
             max_code_bytes = std::max(max_code_bytes, code_bytes_per_warp(ctx, g, split));
         }
+        stage_activations(ctx, items + i0, cnt, p.task);
         p.n_tasks = cnt;
         p.n_units = unit;
         p.split_rows = split ? 1u : 0u;
