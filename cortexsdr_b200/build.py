@@ -15,7 +15,7 @@ SOURCES = [
     "kernels/decode.cu",
     "kernels/gemv_fused.cu",
     "kernels/gemv_queue.cu",
-    "kernels/decoder_ops.cu",
+    "kernels/decoder_ops.cu", "kernels/attention_prompt.cu",
     "kernels/gemm_tcgen05.cu", "kernels/gemm_tma.cu", "kernels/gemm_simt.cu",
     "decoder.cu",
     "kernels/encode.cu",

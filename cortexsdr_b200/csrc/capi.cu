@@ -236,6 +236,7 @@ int csdr_context_create(int device, void* stream, csdr_context** out) {
         if (const char* e = std::getenv("CSDR_TMA")) ctx->tma = e[0] != '0';
         if (const char* e = std::getenv("CSDR_SIMT_MIN_BATCH")) ctx->simt_min_batch = static_cast<size_t>(std::max(1, std::atoi(e)));
         if (const char* e = std::getenv("CSDR_SIMT_MIN_DICT")) ctx->simt_min_dict = static_cast<size_t>(std::max(0, std::atoi(e)));
+        if (const char* e = std::getenv("CSDR_PROMPT_ATTENTION_MIN")) ctx->prompt_attention_min = static_cast<uint32_t>(std::max(1, std::atoi(e)));
         if (const char* e = std::getenv("CSDR_TC_MIN_BATCH")) ctx->tc_min_batch = static_cast<size_t>(std::max(1, std::atoi(e)));
         CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
         *out = ctx.release();

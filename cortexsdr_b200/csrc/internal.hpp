@@ -133,6 +133,7 @@ struct csdr_context {
     bool tma = true;            // CSDR_TMA=0 keeps the register-fed tensor-core kernel
     size_t simt_min_batch = 5;  // CSDR_SIMT_MIN_BATCH: smallest batch of row tiles sent to the fp32 projection instead of the one-launch GEMV
     size_t simt_min_dict = 1u << 18;   // CSDR_SIMT_MIN_DICT: and smallest dictionary (elements), up to sixteen tokens
+    uint32_t prompt_attention_min = 256;  // CSDR_PROMPT_ATTENTION_MIN: shortest prompt whose attention goes block by block
     size_t tc_min_batch = 8;    // CSDR_TC_MIN_BATCH: smallest batch sent to the tcgen05 path
     // Per-device launch facts, remembered per context (function attributes and occupancy belong
     // to a device; a process may hold contexts on several).
