@@ -70,6 +70,14 @@ def _fp(a: np.ndarray):
     return a.ctypes.data_as(C.POINTER(C.c_float))
 
 
+# PyBytes_FromStringAndSize(NULL, n): a bytes object whose memory the library fills before anyone
+# else holds it, so that a payload is not copied once more out of an array.
+_new_bytes = C.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.restype, _new_bytes.argtypes = C.py_object, (C.c_void_p, C.c_ssize_t)
+_bytes_at = C.pythonapi.PyBytes_AsString
+_bytes_at.restype, _bytes_at.argtypes = C.c_void_p, (C.py_object,)
+
+
 def _bytes(b) -> np.ndarray:
     if isinstance(b, np.ndarray):
         return np.ascontiguousarray(b.view(np.uint8).reshape(-1))
@@ -388,9 +396,9 @@ class HierarchicalSDRStrategy:
         rc = lib.csdr_hsdr_encode(*args, None, 0, C.byref(n))
         if rc != _lib.ERR_BUFFER:
             _check(rc)
-        out = np.empty(n.value, np.uint8)
-        _check(lib.csdr_hsdr_encode(*args, out.ctypes.data_as(C.c_void_p), out.size, C.byref(n)))
-        return out.tobytes()
+        out = _new_bytes(None, n.value)
+        _check(lib.csdr_hsdr_encode(*args, _bytes_at(out), n.value, C.byref(n)))
+        return out
 
     def compress_shared(self, tensors, *, tile_rows: int, tile_cols: int, n_atoms: int, n_stages: int = 3, k: int = 8,
                         decay: float = 0.5, ksvd_iters: int = 0):
@@ -412,13 +420,12 @@ class HierarchicalSDRStrategy:
         rc = lib.csdr_hsdr_encode_shared(*head, None, 0, C.byref(dict_n), None, None, code_n)
         if rc != _lib.ERR_BUFFER:
             _check(rc)
-        dict_out = np.empty(dict_n.value, np.uint8)
-        outs = [np.empty(code_n[i], np.uint8) for i in range(n)]
-        out_ptrs = (C.c_void_p * n)(*[o.ctypes.data for o in outs])
-        caps = (C.c_size_t * n)(*[o.size for o in outs])
-        _check(lib.csdr_hsdr_encode_shared(*head, dict_out.ctypes.data_as(C.c_void_p), dict_out.size, C.byref(dict_n), out_ptrs,
-                                           caps, code_n))
-        return dict_out.tobytes(), [o.tobytes() for o in outs]
+        dict_out = _new_bytes(None, dict_n.value)
+        outs = [_new_bytes(None, code_n[i]) for i in range(n)]
+        out_ptrs = (C.c_void_p * n)(*[_bytes_at(o) for o in outs])
+        caps = (C.c_size_t * n)(*[len(o) for o in outs])
+        _check(lib.csdr_hsdr_encode_shared(*head, _bytes_at(dict_out), len(dict_out), C.byref(dict_n), out_ptrs, caps, code_n))
+        return dict_out, outs
 
     def encode_codes(self, tiles, atoms, stage_scales, k: int) -> np.ndarray:
         """The coding pass alone: packed u16 codes (n_tiles, n_stages, k)."""

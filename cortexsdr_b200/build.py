@@ -21,6 +21,7 @@ SOURCES = [
     "kernels/encode.cu",
     "encoder.cu",
     "host/format.cpp",
+    "host/host_copy.cpp",
     "host/archive.cpp",
     "host/sdk_capi.cpp",
 ]

@@ -248,6 +248,7 @@ int csdr_context_destroy(csdr_context* ctx) {
         if (!ctx) return;
         cudaSetDevice(ctx->device);
         cudaStreamSynchronize(ctx->stream);
+        ctx->copier.reset();
         for (auto& s : ctx->scratch) s.reset();
         if (ctx->status_word) cudaFree(ctx->status_word);
         if (ctx->gemv_seq) cudaFree(ctx->gemv_seq);
@@ -914,8 +915,7 @@ int csdr_decompress(csdr_context* ctx, const csdr_segment* seg, float* out_host,
         if (capacity_floats < n) throw Error(CSDR_ERR_BUFFER, "decompress output buffer too small");
         float* dev = static_cast<float*>(ctx->scratch_get(2, n * 4));
         launch_decode_rows(ctx, seg, nullptr, seg->g.rows, dev);
-        CSDR_CUDA(cudaMemcpyAsync(out_host, dev, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
+        ctx->copies().download(out_host, dev, n * 4);
     });
 }
 

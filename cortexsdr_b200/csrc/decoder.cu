@@ -970,14 +970,13 @@ int csdr_decoder_forward(csdr_decoder* d, uint32_t seq, const int32_t* tokens, s
         run_blocks(d, T);
         if (hidden_out) {
             materialise_normed(d, T);
-            CSDR_CUDA(cudaMemcpyAsync(hidden_out, d->normed->ptr, static_cast<size_t>(T) * c.hidden * 4,
-                                      cudaMemcpyDeviceToHost, ctx->stream));
         }
         if (logits_out) {
             run_logits(d, T, T - 1, 1);
             CSDR_CUDA(cudaMemcpyAsync(logits_out, d->logits->ptr, static_cast<size_t>(c.vocab) * 4,
                                       cudaMemcpyDeviceToHost, ctx->stream));
         }
+        if (hidden_out) ctx->copies().download(hidden_out, d->normed->ptr, static_cast<size_t>(T) * c.hidden * 4);
         d->pos_host[seq] = p0 + static_cast<int32_t>(T);
         CSDR_CUDA(cudaMemcpyAsync(I32(d->pos_dev) + seq, &d->pos_host[seq], 4, cudaMemcpyHostToDevice, ctx->stream));
         CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1024,8 +1023,7 @@ int csdr_decoder_step(csdr_decoder* d, const int32_t* tokens, size_t batch, int3
         rethrow_last(csdr_decoder_step_device_async(d, I32(d->tokens_dev), batch, I32(d->next_dev)));
         CSDR_CUDA(cudaMemcpyAsync(next_out, d->next_dev->ptr, batch * 4, cudaMemcpyDeviceToHost, ctx->stream));
         if (logits_out)
-            CSDR_CUDA(cudaMemcpyAsync(logits_out, d->logits->ptr, batch * d->cfg.vocab * 4, cudaMemcpyDeviceToHost,
-                                      ctx->stream));
+            ctx->copies().download(logits_out, d->logits->ptr, batch * d->cfg.vocab * 4);
         CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
     });
 }

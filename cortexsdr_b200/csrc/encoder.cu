@@ -63,18 +63,30 @@ struct Mt19937 {
 void put32(uint8_t* p, uint32_t v) { std::memcpy(p, &v, 4); }
 void put16(uint8_t* p, uint16_t v) { std::memcpy(p, &v, 2); }
 
+// A scratch slot of the context as a buffer object.
+DevPtr scratch(csdr_context* ctx, int slot, size_t bytes) {
+    (void)ctx->scratch_get(slot, bytes);
+    return ctx->scratch[slot];
+}
+
 // fitHierarchicalKSVD (:494-607) on a pool of tiles resident on the device (one tensor's, or the
 // pooled tiles of several tensors as fitSharedDictionary :1446-1469 hands them in): dictionary
 // init, a coding pass, ksvd_iters rounds of (atom update, coding pass), the non-finite sweep.
 void fit_tiles(csdr_context* ctx, const DevPtr& tiles, uint32_t n_tiles, size_t T, uint16_t n_atoms, uint8_t n_stages,
                uint8_t k_per_stage, float stage_decay, uint8_t ksvd_iters, DevPtr* D_out, std::vector<float>* gam_out,
-               DevPtr* codes_out) {
+               const uint16_t** codes_out) {
     const size_t n_codes = static_cast<size_t>(n_tiles) * n_stages * k_per_stage;
+    // the tile norms, picks and stage scales share one block with the codes
+    const size_t picks_at = (static_cast<size_t>(n_tiles) * 8 + 255) & ~static_cast<size_t>(255);
+    const size_t gam_at = (picks_at + static_cast<size_t>(n_atoms) * 4 + 255) & ~static_cast<size_t>(255);
+    const size_t codes_at = (gam_at + 4u * n_stages + 255) & ~static_cast<size_t>(255);
+    const DevPtr small = scratch(ctx, 9, codes_at + n_codes * 2);
+    unsigned char* const small_p = static_cast<unsigned char*>(small->ptr);
     // mean tile norm, summed in tile order on the host from per-tile doubles (:527-533)
-    DevPtr norms = std::make_shared<DeviceBuffer>(static_cast<size_t>(n_tiles) * 8, ctx->device);
-    launch_tile_norms(ctx, static_cast<const float*>(tiles->ptr), n_tiles, static_cast<uint32_t>(T), static_cast<double*>(norms->ptr));
+    double* norms = reinterpret_cast<double*>(small_p);
+    launch_tile_norms(ctx, static_cast<const float*>(tiles->ptr), n_tiles, static_cast<uint32_t>(T), norms);
     std::vector<double> nh(n_tiles);
-    CSDR_CUDA(cudaMemcpyAsync(nh.data(), norms->ptr, nh.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    CSDR_CUDA(cudaMemcpyAsync(nh.data(), norms, nh.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
     CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
     double norm_sum = 0.0;
     for (double v : nh) norm_sum += v;
@@ -86,16 +98,19 @@ void fit_tiles(csdr_context* ctx, const DevPtr& tiles, uint32_t n_tiles, size_t 
     Mt19937 gen(0xC0DEu);
     std::vector<uint32_t> picks(n_atoms);
     for (uint32_t j = 0; j < n_atoms; ++j) picks[j] = gen.below(n_tiles);
-    DevPtr picks_d = upload(ctx, picks.data(), picks.size() * 4);
-    DevPtr D = std::make_shared<DeviceBuffer>(static_cast<size_t>(n_atoms) * T * 4, ctx->device);
-    launch_init_atoms(ctx, static_cast<const float*>(tiles->ptr), static_cast<const uint32_t*>(picks_d->ptr), n_atoms,
+    uint32_t* picks_d = reinterpret_cast<uint32_t*>(small_p + picks_at);
+    CSDR_CUDA(cudaMemcpyAsync(picks_d, picks.data(), picks.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    DevPtr D = scratch(ctx, 8, static_cast<size_t>(n_atoms) * T * 4);
+    D->aux.reset();   // planes of an earlier call's dictionary, had it ended early
+    launch_init_atoms(ctx, static_cast<const float*>(tiles->ptr), picks_d, n_atoms,
                       static_cast<uint32_t>(T), init_scale, static_cast<float*>(D->ptr));
     std::vector<float> gam(n_stages);
     for (uint8_t l = 0; l < n_stages; ++l) gam[l] = std::pow(stage_decay, static_cast<float>(l));   // :507-509
-    DevPtr gam_d = upload(ctx, gam.data(), gam.size() * 4);
-    DevPtr codes = std::make_shared<DeviceBuffer>(n_codes * 2, ctx->device);
+    float* gam_d = reinterpret_cast<float*>(small_p + gam_at);
+    CSDR_CUDA(cudaMemcpyAsync(gam_d, gam.data(), gam.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    uint16_t* codes = reinterpret_cast<uint16_t*>(small_p + codes_at);
     launch_code_tiles(ctx, static_cast<const float*>(tiles->ptr), n_tiles, static_cast<uint32_t>(T), D, n_atoms, n_stages,
-                      k_per_stage, static_cast<const float*>(gam_d->ptr), static_cast<uint16_t*>(codes->ptr));
+                      k_per_stage, gam_d, codes);
     if (ksvd_iters) {
         // the update's target norm (:306-318) from the same tile norms, in double
         const double target = std::max(mean_d / std::sqrt(static_cast<double>(static_cast<uint32_t>(n_stages) * k_per_stage)), 1e-6);
@@ -115,11 +130,11 @@ void fit_tiles(csdr_context* ctx, const DevPtr& tiles, uint32_t n_tiles, size_t 
             CSDR_CUDA(cudaMemcpyAsync(pick_a_d->ptr, pick_a.data(), pick_a.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
             CSDR_CUDA(cudaMemcpyAsync(pick_b_d->ptr, pick_b.data(), pick_b.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
             launch_atom_update(ctx, static_cast<const float*>(tiles->ptr), n_tiles, static_cast<uint32_t>(T),
-                               static_cast<float*>(D->ptr), n_atoms, n_stages, k_per_stage, static_cast<const float*>(gam_d->ptr),
-                               static_cast<const uint16_t*>(codes->ptr), target, static_cast<const uint32_t*>(pick_a_d->ptr),
+                               static_cast<float*>(D->ptr), n_atoms, n_stages, k_per_stage, gam_d,
+                               codes, target, static_cast<const uint32_t*>(pick_a_d->ptr),
                                static_cast<const uint32_t*>(pick_b_d->ptr));
             launch_code_tiles(ctx, static_cast<const float*>(tiles->ptr), n_tiles, static_cast<uint32_t>(T), D, n_atoms, n_stages,
-                              k_per_stage, static_cast<const float*>(gam_d->ptr), static_cast<uint16_t*>(codes->ptr));
+                              k_per_stage, gam_d, codes);
         }
     }
     launch_finite_sweep(ctx, static_cast<float*>(D->ptr), static_cast<size_t>(n_atoms) * T);
@@ -176,12 +191,17 @@ int csdr_hsdr_encode(csdr_context* ctx, const float* W, uint32_t rows, uint32_t 
         if (!payload_out || capacity < total) throw Error(CSDR_ERR_BUFFER, "payload buffer too small");
         uint8_t* out = static_cast<uint8_t*>(payload_out);
 
-        DevPtr Wd = upload(ctx, W, static_cast<size_t>(rows) * cols * 4);
-        DevPtr tiles = std::make_shared<DeviceBuffer>(static_cast<size_t>(n_tiles) * T * 4, ctx->device);
-        launch_extract_tiles(ctx, static_cast<const float*>(Wd->ptr), cols, tile_rows, tile_cols, n_rt, n_ct,
-                             static_cast<float*>(tiles->ptr));
+        DevPtr tiles = scratch(ctx, 2, static_cast<size_t>(rows) * cols * 4);
+        ctx->copies().upload(tiles->ptr, W, static_cast<size_t>(rows) * cols * 4);
+        if (!(tile_rows == 1 && tile_cols == cols)) {   // whole rows are tiles as they lie
+            const DevPtr Wd = tiles;
+            tiles = scratch(ctx, 7, static_cast<size_t>(n_tiles) * T * 4);
+            launch_extract_tiles(ctx, static_cast<const float*>(Wd->ptr), cols, tile_rows, tile_cols, n_rt, n_ct,
+                                 static_cast<float*>(tiles->ptr));
+        }
         std::vector<float> gam;
-        DevPtr D, codes;
+        DevPtr D;
+        const uint16_t* codes = nullptr;
         fit_tiles(ctx, tiles, n_tiles, T, n_atoms, n_stages, k_per_stage, stage_decay, ksvd_iters, &D, &gam, &codes);
 
         // the payload (serialize, :1198-1235): header | stage scales | dictionary | codes | edge strips
@@ -201,9 +221,8 @@ int csdr_hsdr_encode(csdr_context* ctx, const float* W, uint32_t rows, uint32_t 
         std::memcpy(out + hdr, gam.data(), 4u * n_stages);
         uint8_t* dict_at = out + hdr + 4u * n_stages;
         uint8_t* codes_at = dict_at + 4u * static_cast<size_t>(n_atoms) * T;
-        CSDR_CUDA(cudaMemcpyAsync(dict_at, D->ptr, 4u * static_cast<size_t>(n_atoms) * T, cudaMemcpyDeviceToHost, ctx->stream));
-        CSDR_CUDA(cudaMemcpyAsync(codes_at, codes->ptr, n_codes * 2, cudaMemcpyDeviceToHost, ctx->stream));
-        CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
+        ctx->copies().download(dict_at, D->ptr, 4u * static_cast<size_t>(n_atoms) * T);
+        ctx->copies().download(codes_at, codes, n_codes * 2);
         // raw strips: top-right, then bottom (:1185-1197)
         uint8_t* e = codes_at + 2u * n_codes;
         const size_t wr = static_cast<size_t>(cols - C_full) * 4;
@@ -260,12 +279,14 @@ int csdr_hsdr_encode_shared(csdr_context* ctx, const float* const* tensors, cons
             at += static_cast<size_t>(n_rt) * n_ct;
         }
         std::vector<float> gam;
-        DevPtr D, pool_codes;
-        fit_tiles(ctx, pool, n_pool, T, n_atoms, n_stages, k_per_stage, stage_decay, ksvd_iters, &D, &gam, &pool_codes);
+        DevPtr D;
+        const uint16_t* fit_codes = nullptr;
+        fit_tiles(ctx, pool, n_pool, T, n_atoms, n_stages, k_per_stage, stage_decay, ksvd_iters, &D, &gam, &fit_codes);
         // The fit's last step coded the whole pool against the dictionary as it stands before the
         // sweep of non-finite values; the reference codes every tensor again behind the sweep
         // (compressFP32WithExternalDictionary, :2466-2470). One more pass over the pool is that.
         DevPtr gam_d = upload(ctx, gam.data(), gam.size() * 4);
+        DevPtr pool_codes = std::make_shared<DeviceBuffer>(n_pool * slots * 2, ctx->device);
         launch_code_tiles(ctx, static_cast<const float*>(pool->ptr), n_pool, static_cast<uint32_t>(T), D, n_atoms, n_stages, k_per_stage,
                           static_cast<const float*>(gam_d->ptr), static_cast<uint16_t*>(pool_codes->ptr));
 

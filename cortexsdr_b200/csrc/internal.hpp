@@ -12,6 +12,7 @@
 
 #include "../../include/cortexsdr_b200.h"
 #include "host/format.hpp"
+#include "host/host_copy.hpp"
 
 namespace csdr {
 
@@ -100,7 +101,12 @@ struct csdr_context {
     size_t smem_optin = 0;
     uint64_t launches = 0;
     // Grow-only scratch (Dx partials, factored 2-D products, host staging).
-    csdr::DevPtr scratch[8];  // 0 Dx, 1 tile products, 2 materialised W, 3 host staging, 4 fused-GEMV partials, 5 activation planes / wait self-test, 6 GEMV queue, 7 dense product before re-tiling
+    std::unique_ptr<csdr::HostCopier> copier;   // large copies of pageable memory; made on first use
+    csdr::HostCopier& copies() {
+        if (!copier) copier = std::make_unique<csdr::HostCopier>(device, stream);
+        return *copier;
+    }
+    csdr::DevPtr scratch[11];  // 0 Dx, 1 tile products, 2 materialised W, 3 host staging, 4 fused-GEMV partials, 5 activation planes / wait self-test, 6 GEMV queue, 7 dense product before re-tiling, 8 - 10 encoder (dictionary, codes and small arrays, projections)
     void* scratch_get(int slot, size_t bytes);
     int* status_word = nullptr;  // device int: kernels record bounded-wait timeouts here
     // Page-locked, device-mapped host staging for the host-buffer entry points (grow-only).
