@@ -34,6 +34,7 @@
 
 #include "../internal.hpp"
 #include "encode.hpp"
+#include "gemm_simt.hpp"
 #include "gemm_tcgen05.hpp"
 
 namespace csdr {
@@ -89,48 +90,6 @@ init_atoms_kernel(const float* __restrict__ tiles, const uint32_t* __restrict__ 
     const float total = block_sum(sq, red);
     const float norm = sqrtf(fmaxf(total, 1e-24f));
     for (uint32_t c = threadIdx.x; c < T; c += 256) atom[c] = (src[c] / norm) * init_scale;
-}
-
-// C[m][n] = sum_t A[m][t] * B[n][t] on the CUDA cores, for shapes the tensor-core kernel does not
-// take (atoms not a multiple of 128, tile width not a multiple of 8). 64 x 64 tile, 16 x 16 threads.
-constexpr int kTile = 64, kStep = 16;
-__global__ void __launch_bounds__(256) abt_kernel(const float* __restrict__ A, const float* __restrict__ B,
-                                                  float* __restrict__ Cm, uint32_t M, uint32_t N, uint32_t T) {
-    __shared__ float As[kStep][kTile + 1];
-    __shared__ float Bs[kStep][kTile + 1];
-    const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
-    const uint32_t m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
-    float acc[4][4] = {};
-    for (uint32_t t0 = 0; t0 < T; t0 += kStep) {
-        for (uint32_t i = threadIdx.x; i < kTile * kStep; i += 256u) {
-            const uint32_t r = i / kStep, c = i % kStep;
-            const uint32_t t = t0 + c;
-            As[c][r] = (m0 + r < M && t < T) ? A[static_cast<size_t>(m0 + r) * T + t] : 0.f;
-            Bs[c][r] = (n0 + r < N && t < T) ? B[static_cast<size_t>(n0 + r) * T + t] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < kStep; ++c) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a[i] = As[c][ty * 4 + i];
-                b[i] = Bs[c][tx * 4 + i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if (m < M && n < N) Cm[static_cast<size_t>(m) * N + n] = acc[i][j];
-        }
 }
 
 // The greedy rounds. One warp per tile; lane holds the projections on atoms lane + 32 * i.
@@ -426,12 +385,14 @@ void launch_code_tiles(csdr_context* ctx, const float* tiles, uint32_t n_tiles, 
         CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
         D->aux.reset();
     } else {
-        LaunchScope ls(ctx, KC_ENCODE);
-        abt_kernel<<<dim3((n_tiles + kTile - 1) / kTile, (K + kTile - 1) / kTile), 256, 0, ctx->stream>>>(
-            static_cast<const float*>(D->ptr), tiles, Pt, K, n_tiles, T);
-        abt_kernel<<<dim3((K + kTile - 1) / kTile, (K + kTile - 1) / kTile), 256, 0, ctx->stream>>>(
-            static_cast<const float*>(D->ptr), static_cast<const float*>(D->ptr), G, K, K, T);
-        ls.done("abt_kernel");
+        // atom counts and widths the tensor maps do not take: fp32 products (1953 rows of 3492 against
+        // 256 atoms: 1.04 ms for the pass with one 64 x 64 tile a CTA over the whole width)
+        auto dot = [&](const float* rows, uint32_t n, float* out) {
+            launch_gemm_simt(ctx, static_cast<const float*>(D->ptr), K, T, XView{rows, CSDR_DTYPE_F32, CSDR_LAYOUT_TOKEN_MAJOR, T, n, 0u, n},
+                             YView{out, CSDR_LAYOUT_FEATURE_MAJOR, K, n, 0u, n, nullptr}, true);
+        };
+        dot(tiles, n_tiles, Pt);
+        dot(static_cast<const float*>(D->ptr), K, G);
     }
     LaunchScope ls(ctx, KC_ENCODE);
     const dim3 grid((n_tiles + 3u) / 4u);
