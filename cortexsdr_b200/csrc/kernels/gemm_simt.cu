@@ -6,6 +6,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "../internal.hpp"
 #include "gemm_simt.hpp"
@@ -14,13 +15,15 @@ namespace csdr {
 
 namespace {
 
-// Tile of 64 rows x TOK tokens x 32 columns, 128 threads. Both operands lie in shared memory with
+// Tile of 64 rows x TOK (16, 32, 64) tokens x 32 columns, 128 threads. Both operands lie in shared memory with
 // the columns contiguous (36 floats a row: 16-byte aligned, and eight rows cover the 32 banks), so
 // global rows are copied as they are and the inner product runs over pairs of columns on packed
 // fp32 multiply-adds; a thread's 8 x 4 results take 12 128-bit reads per 64 packed instructions.
-// The bound is fp32 issue for 64 tokens and the weight's bytes for 16; small products are bound by
-// the launches. Measured, whole products: 300 atoms of width 350 at 95 tokens 266 -> 21 us (rebuilt
-// weight and a row-a-warp product before), 128 of 2579 at 6 tokens, three members, 441 -> 33 us.
+// Two to four stages in flight. The bound is fp32 issue for 64 tokens (37 TFLOP/s at 11001 x 8100 x
+// 300, half the units' peak; 24 with the addresses worked out per element) and the weight's bytes for
+// 16 (copied four bytes at a time where its width is odd); small products are bound by the launches.
+// Measured, whole products: 300 atoms of width 350 at 95 tokens 266 -> 21 us (rebuilt weight and a
+// row-a-warp product before), 128 of 2579 at 6 tokens, three members, 441 -> 33 us.
 constexpr uint32_t kRows = 64, kCols = 32, kPitch = 36, kThreads = 128;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -43,74 +46,103 @@ struct SimtParams {
     float* part;       // [split][rows][tokens] otherwise
 };
 
-// Copies one 64 x 32 block of W; what lies outside the matrix becomes zero.
-__device__ __forceinline__ void load_w(const SimtParams& p, float* ws, uint32_t row0, uint32_t c0, uint32_t tid) {
-    if (p.vec) {
-#pragma unroll
-        for (uint32_t i = 0; i < kRows * kCols / 4u / kThreads; ++i) {
-            const uint32_t e = tid + i * kThreads, r = e >> 3, c = (e & 7u) * 4u;
-            const bool in = row0 + r < p.rows && c0 + c < p.cols;   // cols is a multiple of four
-            const float* src = in ? p.W + static_cast<size_t>(row0 + r) * p.cols + c0 + c : p.W;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(ws + r * kPitch + c)), "l"(src),
-                         "r"(in ? 16u : 0u)
-                         : "memory");
-        }
-    } else {
-#pragma unroll
-        for (uint32_t i = 0; i < kRows * kCols / kThreads; ++i) {
-            const uint32_t e = tid + i * kThreads, r = e >> 5, c = e & 31u;
-            const bool in = row0 + r < p.rows && c0 + c < p.cols;
-            const float* src = in ? p.W + static_cast<size_t>(row0 + r) * p.cols + c0 + c : p.W;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(ws + r * kPitch + c)), "l"(src),
-                         "r"(in ? 4u : 0u)
-                         : "memory");
-        }
+// A thread's share of the 64 x 32 blocks of W: where its copies come from and go to, fixed but for
+// the column. What lies outside the matrix becomes zero.
+struct WBlock {
+    const float* src;      // of the first copy at column 0
+    uint32_t dst, c, rows_in;
+    __device__ __forceinline__ WBlock(const SimtParams& p, uint32_t row0, uint32_t tid) {
+        const uint32_t r = p.vec ? tid >> 3 : tid >> 5;
+        c = p.vec ? (tid & 7u) * 4u : tid & 31u;
+        src = p.W + static_cast<size_t>(row0 + r) * p.cols + c;
+        dst = (r * kPitch + c) * 4u;
+        rows_in = p.rows > row0 + r ? p.rows - row0 - r : 0u;     // rows of the matrix from this copy's on
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-// A thread's share of a TOK x 32 block of the activations, in registers: lanes run along whichever
-// of the two dimensions is contiguous in memory.
-template <uint32_t TOK>
-struct XBlock {
-    static constexpr uint32_t N = TOK * kCols / kThreads;
-    float v[N];
-    __device__ __forceinline__ static void at(const SimtParams& p, uint32_t e, uint32_t& t, uint32_t& c) {
-        if (p.x.layout == CSDR_LAYOUT_FEATURE_MAJOR) {
-            t = e % TOK;
-            c = e / TOK;
+    __device__ __forceinline__ void load(const SimtParams& p, const float* ws, uint32_t c0) const {
+        const uint32_t base = smem_u32(ws) + dst;
+        const bool col = c0 + c < p.cols;
+        if (p.vec) {   // cols is a multiple of four
+            constexpr uint32_t step = kThreads / 8u;
+#pragma unroll
+            for (uint32_t i = 0; i < kRows / step; ++i) {
+                const bool in = col && i * step < rows_in;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + i * step * kPitch * 4u),
+                             "l"(in ? src + c0 + static_cast<size_t>(i) * step * p.cols : p.W), "r"(in ? 16u : 0u)
+                             : "memory");
+            }
         } else {
-            t = e / kCols;
-            c = e % kCols;
-        }
-    }
-    __device__ __forceinline__ void load(const SimtParams& p, uint32_t t0, uint32_t c0, uint32_t tid) {
+            constexpr uint32_t step = kThreads / 32u;
 #pragma unroll
-        for (uint32_t i = 0; i < N; ++i) {
-            uint32_t t, c;
-            at(p, tid + i * kThreads, t, c);
-            v[i] = t0 + t < p.x.M && c0 + c < p.cols ? load_x(p.x, c0 + c, t0 + t) : 0.0f;
-        }
-    }
-    __device__ __forceinline__ void store(const SimtParams& p, float* xs, uint32_t tid) const {
-#pragma unroll
-        for (uint32_t i = 0; i < N; ++i) {
-            uint32_t t, c;
-            at(p, tid + i * kThreads, t, c);
-            xs[t * kPitch + c] = v[i];
+            for (uint32_t i = 0; i < kRows / step; ++i) {
+                const bool in = col && i * step < rows_in;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(base + i * step * kPitch * 4u),
+                             "l"(in ? src + c0 + static_cast<size_t>(i) * step * p.cols : p.W), "r"(in ? 4u : 0u)
+                             : "memory");
+            }
         }
     }
 };
 
+// A thread's share of the TOK x 32 blocks of the activations: lanes run along whichever of the two
+// dimensions is contiguous in memory. fp32 is copied asynchronously like W; bf16 is widened on its
+// way through registers.
+template <uint32_t TOK, typename X, bool FEATURE_MAJOR>
+struct XBlock {
+    static constexpr uint32_t N = TOK * kCols / kThreads;
+    static constexpr uint32_t step_t = FEATURE_MAJOR ? 0u : kThreads / kCols, step_c = FEATURE_MAJOR ? kThreads / TOK : 0u;
+    const X* src;
+    uint32_t t, c, toks_in;
+    size_t stride;         // between this thread's elements; col: between neighbouring columns
+    size_t col;
+    float v[N];
+    __device__ __forceinline__ XBlock(const SimtParams& p, uint32_t t0, uint32_t tid) {
+        t = FEATURE_MAJOR ? tid % TOK : tid / kCols;
+        c = FEATURE_MAJOR ? tid / TOK : tid % kCols;
+        const size_t tok = FEATURE_MAJOR ? 1u : p.x.C;
+        col = FEATURE_MAJOR ? p.x.Mtotal : 1u;
+        src = static_cast<const X*>(p.x.x) + (p.x.b0 + t0 + t) * tok + c * col;
+        stride = step_t * tok + step_c * col;
+        toks_in = p.x.M > t0 + t ? p.x.M - t0 - t : 0u;
+    }
+    __device__ __forceinline__ void load(const SimtParams& p, uint32_t c0) {
+        const X* at = src + c0 * col;
+        const uint32_t cols_in = p.cols > c0 + c ? p.cols - c0 - c : 0u;
+#pragma unroll
+        for (uint32_t i = 0; i < N; ++i)
+            v[i] = i * step_t < toks_in && i * step_c < cols_in ? static_cast<float>(at[i * stride]) : 0.0f;
+    }
+    __device__ __forceinline__ void load_async(const SimtParams& p, const float* xs, uint32_t c0) const {
+        const X* at = src + c0 * col;
+        const uint32_t cols_in = p.cols > c0 + c ? p.cols - c0 - c : 0u;
+        const uint32_t base = smem_u32(xs) + (t * kPitch + c) * 4u;
+#pragma unroll
+        for (uint32_t i = 0; i < N; ++i) {
+            const bool in = i * step_t < toks_in && i * step_c < cols_in;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(base + (i * step_t * kPitch + i * step_c) * 4u),
+                         "l"(in ? static_cast<const void*>(at + i * stride) : p.x.x), "r"(in ? 4u : 0u)
+                         : "memory");
+        }
+    }
+    __device__ __forceinline__ void store(float* xs) const {
+#pragma unroll
+        for (uint32_t i = 0; i < N; ++i) xs[(t + i * step_t) * kPitch + c + i * step_c] = v[i];
+    }
+};
+
+template <uint32_t TOK>
+constexpr uint32_t stages() { return TOK == 64u ? 2u : TOK == 32u ? 3u : 4u; }   // all that static shared memory holds
+
 // grid (row tiles, token tiles, column ranges). SWAP: lanes run along the rows of W instead of the
 // tokens, so that a token-major result leaves in contiguous pieces.
-template <uint32_t TOK, bool SWAP>
-__global__ void __launch_bounds__(kThreads)
+template <uint32_t TOK, bool SWAP, typename X, bool FEATURE_MAJOR>
+__global__ void __launch_bounds__(kThreads, 3)
 hsdr_gemm_simt_kernel(const __grid_constant__ SimtParams p) {
-    __shared__ __align__(16) float ws[2][kRows * kPitch];
-    __shared__ __align__(16) float xs[2][TOK * kPitch];
+    constexpr uint32_t NS = stages<TOK>();
+    constexpr bool ASYNC_X = sizeof(X) == 4u;
+    __shared__ __align__(16) float ws[NS][kRows * kPitch];
+    __shared__ __align__(16) float xs[NS][TOK * kPitch];
     constexpr uint32_t A = SWAP ? TOK : kRows, B = SWAP ? kRows : TOK;   // slow and fast dimension of the result
-    constexpr uint32_t TB = B >= 64u ? 16u : 8u, TA = kThreads / TB;     // threads along each
+    constexpr uint32_t TB = B >= 32u ? 16u : 8u, TA = kThreads / TB;     // threads along each
     constexpr uint32_t NA = A / TA, NB = B / TB;
     const uint32_t tid = threadIdx.x, tb = tid % TB, ta = tid / TB;
     const uint32_t row0 = blockIdx.x * kRows, t0 = blockIdx.y * TOK;
@@ -120,24 +152,34 @@ hsdr_gemm_simt_kernel(const __grid_constant__ SimtParams p) {
     for (uint32_t i = 0; i < NA; ++i)
 #pragma unroll
         for (uint32_t j = 0; j < NB; ++j) acc[i][j] = 0ull;
-    XBlock<TOK> xb;
+    const WBlock wb(p, row0, tid);
+    XBlock<TOK, X, FEATURE_MAJOR> xb(p, t0, tid);
     // a resident weight is no other launch's output; a rebuilt one and the activations may be
     if (p.w_fresh) asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (kb0 < kb1) load_w(p, ws[0], row0, kb0 * kCols, tid);
+#pragma unroll
+    for (uint32_t i = 0; i + 1u < NS; ++i)
+        if (kb0 + i < kb1) wb.load(p, ws[i], (kb0 + i) * kCols);
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (kb0 < kb1) {
-        xb.load(p, t0, kb0 * kCols, tid);
-        xb.store(p, xs[0], tid);
+#pragma unroll
+    for (uint32_t i = 0; i + 1u < NS; ++i) {   // the first group covers every copy of W so far
+        if (ASYNC_X && kb0 + i < kb1) xb.load_async(p, xs[i], (kb0 + i) * kCols);
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    if (!ASYNC_X && kb0 < kb1) {
+        xb.load(p, kb0 * kCols);
+        xb.store(xs[0]);
+    }
+    uint32_t s = 0;
     for (uint32_t kb = kb0; kb < kb1; ++kb) {
-        const uint32_t s = (kb - kb0) & 1u;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        const bool more = kb + 1u < kb1;
-        if (more) {
-            load_w(p, ws[s ^ 1u], row0, (kb + 1u) * kCols, tid);
-            xb.load(p, t0, (kb + 1u) * kCols, tid);
+        asm volatile("cp.async.wait_group %0;" ::"n"(static_cast<int>(NS) - 2) : "memory");
+        __syncthreads();                       // block kb is here, and block kb - 1 has been read
+        const uint32_t next = s + 1u == NS ? 0u : s + 1u, ahead = s == 0u ? NS - 1u : s - 1u;
+        if (kb + NS - 1u < kb1) {
+            wb.load(p, ws[ahead], (kb + NS - 1u) * kCols);
+            if (ASYNC_X) xb.load_async(p, xs[ahead], (kb + NS - 1u) * kCols);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (!ASYNC_X && kb + 1u < kb1) xb.load(p, (kb + 1u) * kCols);
         const float* as = (SWAP ? xs[s] : ws[s]) + ta * kPitch;
         const float* bs = (SWAP ? ws[s] : xs[s]) + tb * kPitch;
 #pragma unroll 2
@@ -152,7 +194,8 @@ hsdr_gemm_simt_kernel(const __grid_constant__ SimtParams p) {
 #pragma unroll
                 for (uint32_t j = 0; j < NB; ++j) acc[i][j] = fma2(a[i].y, b[j].y, fma2(a[i].x, b[j].x, acc[i][j]));
         }
-        if (more) xb.store(p, xs[s ^ 1u], tid);   // the other buffer: its readers met the barrier above
+        if (!ASYNC_X && kb + 1u < kb1) xb.store(xs[next]);
+        s = next;
     }
     asm volatile("griddepcontrol.launch_dependents;");
 #pragma unroll
@@ -199,9 +242,8 @@ simt_reduce_kernel(const float* __restrict__ part, uint32_t rows, uint32_t M, ui
 void launch_gemm_simt(csdr_context* ctx, const float* W, uint32_t rows, uint32_t cols, const XView& x, const YView& y,
                       bool w_fresh) {
     if (rows == 0 || x.M == 0) return;
-    const bool narrow = x.M <= 16u;
     const bool swap = y.layout == CSDR_LAYOUT_TOKEN_MAJOR;
-    const uint32_t tok = narrow ? 16u : 64u;
+    const uint32_t tok = x.M <= 16u ? 16u : x.M <= 32u ? 32u : 64u;
     SimtParams p{};
     p.W = W;
     p.rows = rows;
@@ -232,8 +274,16 @@ void launch_gemm_simt(csdr_context* ctx, const float* W, uint32_t rows, uint32_t
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     {
-        auto kern = narrow ? (swap ? hsdr_gemm_simt_kernel<16, true> : hsdr_gemm_simt_kernel<16, false>)
-                           : (swap ? hsdr_gemm_simt_kernel<64, true> : hsdr_gemm_simt_kernel<64, false>);
+        auto pick = [&](auto type, auto fm) {
+            using X = decltype(type);
+            constexpr bool FM = decltype(fm)::value;
+            return tok == 16u ? (swap ? hsdr_gemm_simt_kernel<16, true, X, FM> : hsdr_gemm_simt_kernel<16, false, X, FM>)
+                   : tok == 32u ? (swap ? hsdr_gemm_simt_kernel<32, true, X, FM> : hsdr_gemm_simt_kernel<32, false, X, FM>)
+                          : (swap ? hsdr_gemm_simt_kernel<64, true, X, FM> : hsdr_gemm_simt_kernel<64, false, X, FM>);
+        };
+        const bool fm = x.layout == CSDR_LAYOUT_FEATURE_MAJOR;
+        auto kern = x.dtype == CSDR_DTYPE_BF16 ? (fm ? pick(__nv_bfloat16{}, std::true_type{}) : pick(__nv_bfloat16{}, std::false_type{}))
+                                               : (fm ? pick(float{}, std::true_type{}) : pick(float{}, std::false_type{}));
         LaunchScope ls(ctx, KC_DX);
         CSDR_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
         ls.done("hsdr_gemm_simt_kernel");

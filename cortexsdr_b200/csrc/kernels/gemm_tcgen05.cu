@@ -1188,10 +1188,10 @@ void launch_matmul_tcgen05(csdr_context* ctx, const csdr_segment* seg, const Mat
 
 // Widths that are no multiple of four have no 128-bit rows: Dx comes from the fp32 product at any
 // batch, and the gathers above read it. Others leave the one-launch GEMV from five tokens on where
-// the dictionary is larger than 2^18 elements (512 atoms of 4096 at 5 tokens: 18.4 against 15.0 us,
-// 300 of 1024: 10.4 against 9.3; 128 of 2048, the size of the line: 10.1 against 11.0 at 5 tokens,
-// 10.2 against 9.4 at 7; 300 of 512, below it: 8.0 against 13.8; up to four tokens 512 of 4096: 11.8
-// against 13.6), and past its sixteen tokens always. The bounds are the gathers' shared memory.
+// the dictionary has at least 2^18 elements (512 atoms of 4096 at 5 tokens: 18.3 against 14.7 us, 300
+// of 1024: 10.4 against 9.2, 128 of 2048: 9.9 against 9.1; 300 of 512, below the line: 8.1 against
+// 13.4; up to four tokens 512 of 4096: 11.8 against 12.7), and past its sixteen tokens always. The
+// bounds are the gathers' shared memory.
 bool simt_rows_supported(const csdr_context* ctx, const csdr_segment* seg, size_t batch) {
     const Geometry& g = seg->g;
     if (!g.row_tiles() || batch > 0xFFFFFFFFull || g.slots() > kWideMaxSlots || g.n_stages > 64u) return false;

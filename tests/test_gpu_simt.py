@@ -39,6 +39,7 @@ def product(ctx, pay, x, dtype, token, bias=None):
     (300, 1021, 0, 300, 8, 5),      # column ranges, odd width
     (300, 1024, 0, 300, 5, 16),     # aligned rows, widest narrow tile
     (129, 514, 0, 128, 8, 17),      # one token past the narrow tile; width 2 mod 4
+    (90, 2050, 0, 100, 8, 32),      # the middle token tile exactly, several blocks a range
     (64, 1000, 0, 129, 4, 64),      # a token tile exactly
     (513, 333, 0, 40, 8, 131),      # ragged in every direction
     (100, 100, 16, 20, 4, 3),       # tiles with both strips, few tokens
