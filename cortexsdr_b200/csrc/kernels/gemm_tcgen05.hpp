@@ -28,6 +28,11 @@ void launch_dx_tma(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs&
 // Builds and caches the bf16 planes of the segment's dictionary now (they are otherwise built
 // on the first projection); afterwards the fp32 atoms are no longer read by the TMA kernel.
 void dx_tma_prepare(csdr_context* ctx, const csdr_segment* seg);
+// All tile products of a 2-D tile segment for x.M tokens: tile_view is its dictionary seen as n_atoms *
+// tile_rows rows of tile_cols columns; out is [token * n_ct + column tile][that many rows].
+struct XView;
+bool tile_project_supported(const csdr_context* ctx, const csdr_segment* tile_view, size_t n_tok, bool x_has_lo);
+void launch_tile_project(csdr_context* ctx, const csdr_segment* tile_view, const XView& x, uint32_t n_ct, float* out);
 
 
 // Activations as token-major bf16 planes [tokens][cols]: hi = bf16(x), lo = bf16(x - hi); lo is

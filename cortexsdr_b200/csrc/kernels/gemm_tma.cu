@@ -440,6 +440,9 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
         const uint32_t n4 = N / 4u;
         const bool vec = ((p.M | p.dx_stride) & 3u) == 0;
         const float* tile_part = p.part + static_cast<size_t>(tile) * n_ranks * kTileM * N;
+        // neighbouring threads take neighbouring pieces of what is contiguous on the way out
+        auto row_of = [&](uint32_t i) { return p.transposed ? i % rows_mine : i / n4; };
+        auto c4_of = [&](uint32_t i) { return p.transposed ? i / rows_mine : i % n4; };
         // two items per pass, every rank's piece of both requested before the first add: the
         // loads are L2 round trips and must overlap
         for (uint32_t i0 = tid; i0 < rows_mine * n4; i0 += 2u * kThreads) {
@@ -448,7 +451,7 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
             for (uint32_t h = 0; h < 2u; ++h) {
                 const uint32_t i = i0 + h * kThreads;
                 if (i < rows_mine * n4) {
-                    const uint32_t row = row_begin + i / n4, c4 = i % n4;
+                    const uint32_t row = row_begin + row_of(i), c4 = c4_of(i);
                     const float* src = tile_part + static_cast<size_t>(row) * N + c4 * 4u;
 #pragma unroll
                     for (uint32_t r = 0; r < 16u; ++r)
@@ -460,7 +463,7 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
             for (uint32_t h = 0; h < 2u; ++h) {
                 const uint32_t i = i0 + h * kThreads;
                 if (i >= rows_mine * n4) break;
-                const uint32_t row = row_begin + i / n4, c4 = i % n4;
+                const uint32_t row = row_begin + row_of(i), c4 = c4_of(i);
                 float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (uint32_t r = 0; r < 16u; ++r)
@@ -499,6 +502,183 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
         }
     }
     __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tmem_cols) : "memory");
+    }
+}
+
+// ---- tile products of 2-D tiles: P_T[token * n_ct + column tile][atom * Tr + row] ----
+// The dictionary read as K * Tr rows of Tc columns against batch * n_ct column tiles of the
+// activations: many row tiles (512 for 512 atoms of 128 x 128), each only one or two 64-column blocks
+// deep. With a CTA per row tile (hsdr_dx_tma_kernel) setting up barriers, tensor memory and the
+// activation planes cost more than the products: 22 us for 33 MB of planes. Here a CTA stays and walks
+// row tiles: its activations are split into bf16 hi / lo once, straight from the caller's matrix into
+// the MMA's layout, the ring of weight blocks runs on across row tiles, and two accumulators let the
+// epilogue of one tile (tensor memory lanes are rows, so a warp stores 128 contiguous bytes of a
+// token's row) overlap the products of the next. Same products in the same order as before.
+constexpr uint32_t kTileStages = 5;
+
+struct TileProjectParams {
+    XView x;
+    float* out;              // [n_tok][rows]
+    uint32_t rows;           // K * Tr, a multiple of 128
+    uint32_t Tc, n_ct, n_tok;
+    uint32_t n_tile, n_kb, stages;
+    uint32_t x_has_lo;
+    uint32_t tmem_cols;
+    int* status;
+    uint32_t spin;
+};
+
+// grid (CTAs over the row tiles, token tiles)
+__global__ void __launch_bounds__(kThreads, 1)
+hsdr_tile_project_mma_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
+                             const __grid_constant__ TileProjectParams p) {
+    extern __shared__ __align__(1024) unsigned char tma_smem_raw[];
+    asm volatile("griddepcontrol.launch_dependents;");
+    __shared__ __align__(8) unsigned long long full_bar[kTileStages], empty_bar[kTileStages], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_base_s;
+    __shared__ volatile int failed_s;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    unsigned char* smem = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(tma_smem_raw) + 1023u) & ~static_cast<uintptr_t>(1023));
+    const uint32_t N = p.n_tile, b_tile = N * 128u, x_planes = p.x_has_lo ? 2u : 1u;
+    unsigned char* xs = smem;                                        // [kb][plane][N][128 B], swizzled
+    unsigned char* ring = smem + p.n_kb * x_planes * b_tile;         // [stage][hi | lo][128][128 B]
+    constexpr uint32_t stage_bytes = 2u * kATile;
+    const uint32_t n_tiles = p.rows / kTileM, tok0 = blockIdx.y * N;
+    const uint32_t mine = blockIdx.x < n_tiles ? (n_tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
+    const uint32_t n_it = mine * p.n_kb;
+    if (tid == 0) {
+        for (uint32_t i = 0; i < kTileStages; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full_bar[i])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty_bar[i])));
+        }
+        for (uint32_t i = 0; i < 2u; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&acc_full[i])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(smem_u32(&acc_empty[i])));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        failed_s = 0;
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
+                     "r"(p.tmem_cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    __syncthreads();
+    auto load = [&](uint32_t it) {      // weight block it of this CTA's walk: nobody else's output, read ahead
+        const uint32_t s = it % p.stages, tile = blockIdx.x + it / p.n_kb * gridDim.x, kb = it % p.n_kb;
+        const uint32_t bar = smem_u32(&full_bar[s]), dst = smem_u32(ring + s * stage_bytes);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(stage_bytes) : "memory");
+        tma_load_2d(dst, &map_hi, kb * kBlockK, tile * kTileM, bar);
+        tma_load_2d(dst + kATile, &map_lo, kb * kBlockK, tile * kTileM, bar);
+    };
+    const uint32_t pre = min(p.stages, n_it);
+    if (tid == 0)
+        for (uint32_t it = 0; it < pre; ++it) load(it);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // activations: eight columns of one (token, column tile) at a time, one 16-byte unit of the
+    // 128-byte swizzled rows; columns past the tile and tokens past the end are zero
+    for (uint32_t i = tid; i < p.n_kb * N * 8u; i += kThreads) {
+        const uint32_t kb = i / (N * 8u), r = i - kb * N * 8u, t = r >> 3, u = r & 7u;
+        const uint32_t tok = tok0 + t, c0 = kb * kBlockK + u * 8u;
+        alignas(16) __nv_bfloat16 h[8], l[8];
+#pragma unroll
+        for (uint32_t e = 0; e < 8u; ++e) {
+            float v = 0.0f;
+            if (tok < p.n_tok && c0 + e < p.Tc) {
+                const uint32_t b = tok / p.n_ct, bc = tok - b * p.n_ct;
+                v = load_x(p.x, bc * p.Tc + c0 + e, b);
+            }
+            h[e] = __float2bfloat16_rn(v);
+            l[e] = __float2bfloat16_rn(v - __bfloat162float(h[e]));
+        }
+        unsigned char* dst = xs + kb * x_planes * b_tile + (t >> 3) * 1024u + (t & 7u) * 128u + ((u ^ (t & 7u)) << 4);
+        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(h);
+        if (p.x_has_lo) *reinterpret_cast<uint4*>(dst + b_tile) = *reinterpret_cast<const uint4*>(l);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the MMAs read what was just stored
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = tmem_base_s;
+    if (warp == 0) {
+        if (lane == 0)
+            for (uint32_t it = pre; it < n_it; ++it) {
+                if (!mbar_wait(smem_u32(&empty_bar[it % p.stages]), (it / p.stages - 1u) & 1u, p.spin)) failed_s = 1;
+                if (failed_s) break;
+                load(it);
+            }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc(N);
+            bool ok = true;
+            for (uint32_t ti = 0; ti < mine && ok; ++ti) {
+                const uint32_t acc = ti & 1u, d = tmem_base + acc * N;
+                if (ti >= 2u) ok = mbar_wait(smem_u32(&acc_empty[acc]), (ti / 2u - 1u) & 1u, p.spin);
+                for (uint32_t kb = 0; kb < p.n_kb && ok; ++kb) {
+                    const uint32_t it = ti * p.n_kb + kb, s = it % p.stages;
+                    ok = mbar_wait(smem_u32(&full_bar[s]), (it / p.stages) & 1u, p.spin) && !failed_s;
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t a_hi = smem_u32(ring + s * stage_bytes), a_lo = a_hi + kATile;
+                    const uint32_t b_hi = smem_u32(xs + kb * x_planes * b_tile), b_lo = b_hi + b_tile;
+#pragma unroll
+                    for (uint32_t k = 0; k < kBlockK / 16u; ++k) {
+                        const uint64_t ah = make_desc(a_hi + k * 32u), al = make_desc(a_lo + k * 32u);
+                        const uint64_t bh = make_desc(b_hi + k * 32u);
+                        mma_bf16(d, ah, bh, idesc, (kb | k) != 0u);
+                        mma_bf16(d, al, bh, idesc, 1u);
+                        if (p.x_has_lo) mma_bf16(d, ah, make_desc(b_lo + k * 32u), idesc, 1u);
+                    }
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                     smem_u32(&empty_bar[s]))
+                                 : "memory");
+                }
+                if (ok)
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                     smem_u32(&acc_full[acc]))
+                                 : "memory");
+            }
+            if (!ok) failed_s = 1;
+        }
+    } else {
+        const uint32_t quad = warp & 3u, row = quad * 32u + lane;
+        for (uint32_t ti = 0; ti < mine; ++ti) {
+            const uint32_t acc = ti & 1u;
+            const bool ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&acc_full[acc]), (ti / 2u) & 1u, p.spin));
+            if (!ok) {
+                failed_s = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            float* dst = p.out + static_cast<size_t>(tok0) * p.rows + (blockIdx.x + ti * gridDim.x) * kTileM + row;
+            for (uint32_t ch = 0; ch < N / 16u; ++ch) {
+                uint32_t r[16];
+                const uint32_t taddr = tmem_base + acc * N + ((quad * 32u) << 16) + ch * 16u;
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+                      "=r"(r[15])
+                    : "r"(taddr)
+                    : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (uint32_t j = 0; j < 16u; ++j)
+                    if (tok0 + ch * 16u + j < p.n_tok) dst[static_cast<size_t>(ch * 16u + j) * p.rows] = __uint_as_float(r[j]);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[acc])) : "memory");
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (tid == 0 && failed_s) atomicExch(p.status, 1);
     if (warp == 1) {
         __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tmem_cols) : "memory");
@@ -757,6 +937,57 @@ void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uin
     LaunchScope ls(ctx, KC_GEMM);
     CSDR_CUDA(cudaLaunchKernelEx(&cfg, hsdr_dx_tma_kernel, maps, map_xhi, map_xlo, p));
     ls.done("hsdr_dx_tma_kernel");
+}
+
+// Shared memory beside the barriers: the activations of a token tile and the ring of weight blocks.
+// At least three stages must fit, else the plain projection computes the tile products.
+bool tile_project_supported(const csdr_context* ctx, const csdr_segment* tile_view, size_t n_tok, bool x_has_lo) {
+    using namespace tma_detail;
+    if (!dx_tma_supported(ctx, tile_view, n_tok) || n_tok == 0 || n_tok > 0x7FFFFFFFu) return false;
+    const uint32_t n_kb = (tile_view->g.cols + kBlockK - 1u) / kBlockK;
+    uint32_t N = 16;
+    while (N < 128u && N < n_tok) N <<= 1;
+    return static_cast<size_t>(n_kb) * (x_has_lo ? 2u : 1u) * N * 128u + 3u * 2u * kATile + 4096u <= ctx->smem_optin;
+}
+
+void launch_tile_project(csdr_context* ctx, const csdr_segment* tile_view, const XView& x, uint32_t n_ct, float* out) {
+    using namespace tma_detail;
+    const auto planes = planes_for(ctx, tile_view);
+    const Geometry& g = tile_view->g;
+    TileProjectParams p{};
+    p.x = x;
+    p.out = out;
+    p.rows = g.n_atoms;
+    p.Tc = g.cols;
+    p.n_ct = n_ct;
+    p.n_tok = x.M * n_ct;
+    p.n_tile = 16;
+    while (p.n_tile < 128u && p.n_tile < p.n_tok) p.n_tile <<= 1;
+    p.n_kb = (g.cols + kBlockK - 1u) / kBlockK;
+    p.x_has_lo = x.dtype == CSDR_DTYPE_F32 ? 1u : 0u;
+    p.tmem_cols = std::max(32u, 2u * p.n_tile);
+    const size_t x_bytes = static_cast<size_t>(p.n_kb) * (p.x_has_lo ? 2u : 1u) * p.n_tile * 128u;
+    const size_t smem_max = ctx->smem_optin - 2048u;
+    p.stages = static_cast<uint32_t>(std::min<size_t>(kTileStages, (smem_max - 1024u - x_bytes) / (2u * kATile)));
+    const size_t smem = x_bytes + static_cast<size_t>(p.stages) * 2u * kATile + 1024u;
+    p.status = ctx->status_word;
+    p.spin = ctx->spin_limit_barrier;
+    ctx->opt_in_smem(reinterpret_cast<const void*>(hsdr_tile_project_mma_kernel), smem);
+    const uint32_t tok_tiles = (p.n_tok + p.n_tile - 1u) / p.n_tile, tiles = p.rows / kTileM;
+    const uint32_t per = std::max(1u, static_cast<uint32_t>(ctx->sm_count) / tok_tiles);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(std::min(tiles, per), tok_tiles, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    LaunchScope ls(ctx, KC_GEMM);
+    CSDR_CUDA(cudaLaunchKernelEx(&cfg, hsdr_tile_project_mma_kernel, planes->map_hi, planes->map_lo, p));
+    ls.done("hsdr_tile_project_mma_kernel");
 }
 
 void dx_tma_prepare(csdr_context* ctx, const csdr_segment* seg) { (void)tma_detail::planes_for(ctx, seg); }
