@@ -16,7 +16,7 @@ SOURCES = [
     "kernels/gemv_fused.cu",
     "kernels/gemv_queue.cu",
     "kernels/decoder_ops.cu", "kernels/attention_prompt.cu",
-    "kernels/gemm_tcgen05.cu", "kernels/gemm_tma.cu", "kernels/gemm_simt.cu",
+    "kernels/gemm_tcgen05.cu", "kernels/gemm_tma.cu", "kernels/gemm_simt.cu", "kernels/gather_mma.cu",
     "decoder.cu",
     "kernels/encode.cu",
     "encoder.cu",

@@ -234,6 +234,8 @@ int csdr_context_create(int device, void* stream, csdr_context** out) {
         if (const char* e = std::getenv("CSDR_PDL")) ctx->pdl = e[0] != '0';
         if (const char* e = std::getenv("CSDR_TENSOR_CORES")) ctx->tensor_cores = e[0] != '0';
         if (const char* e = std::getenv("CSDR_TMA")) ctx->tma = e[0] != '0';
+        if (const char* e = std::getenv("CSDR_GATHER_MMA")) ctx->gather_mma = e[0] != '0';
+        if (const char* e = std::getenv("CSDR_GATHER_MMA_MIN")) ctx->gather_mma_min = static_cast<size_t>(std::max(0, std::atoi(e)));
         if (const char* e = std::getenv("CSDR_SIMT_MIN_BATCH")) ctx->simt_min_batch = static_cast<size_t>(std::max(1, std::atoi(e)));
         if (const char* e = std::getenv("CSDR_SIMT_MIN_DICT")) ctx->simt_min_dict = static_cast<size_t>(std::max(0, std::atoi(e)));
         if (const char* e = std::getenv("CSDR_PROMPT_ATTENTION_MIN")) ctx->prompt_attention_min = static_cast<uint32_t>(std::max(1, std::atoi(e)));

@@ -376,7 +376,7 @@ bool wide(csdr_decoder* d, std::initializer_list<const Linear*> ls, const __nv_b
         gather(w);
         return false;
     }
-    const WideDx w = launch_wide_project(d->ctx, segs, n, xp, T, base + d->sum_pad, nullptr, nullptr, nullptr, &shares);
+    const WideDx w = launch_wide_project(d->ctx, segs, n, xp, T, base + d->sum_pad, nullptr, nullptr, nullptr, &shares, partial && d->P > 1);
     if (partial) sum_over_ranks(d, w.base, w.floats);
     if (act_hi && w.tile_mt) {
         launch_wide_gather_swiglu(d->ctx, segs, w, T, ts, act_hi, act_lo);

@@ -137,6 +137,8 @@ struct csdr_context {
     bool pdl = true;         // CSDR_PDL=0 launches without programmatic dependent launch
     bool tensor_cores = true;   // CSDR_TENSOR_CORES=0 keeps wide batches on the CUDA-core kernels
     bool tma = true;            // CSDR_TMA=0 keeps the register-fed tensor-core kernel
+    bool gather_mma = true;     // CSDR_GATHER_MMA=0 keeps wide gathers on shared-memory lookups
+    size_t gather_mma_min = 0;  // CSDR_GATHER_MMA_MIN: smallest batch (17 and up) whose gather goes to the tensor cores; 0: by size
     size_t simt_min_batch = 5;  // CSDR_SIMT_MIN_BATCH: smallest batch of row tiles sent to the fp32 projection instead of the one-launch GEMV
     size_t simt_min_dict = 1u << 18;   // CSDR_SIMT_MIN_DICT: and smallest dictionary (elements), up to sixteen tokens
     uint32_t prompt_attention_min = 256;  // CSDR_PROMPT_ATTENTION_MIN: shortest prompt whose attention goes block by block
@@ -178,6 +180,8 @@ struct csdr_segment {
     // 2-D tile images only: the dictionary seen as n_atoms * tile_rows rows of tile_cols columns,
     // the shape in which the tensor-core projection computes all tile products of a few tokens.
     mutable std::shared_ptr<csdr_segment> tile_view;
+    // Row tiles: the codes as coefficient entries sorted by row tile and atom block (gather_mma.cu).
+    mutable csdr::DevPtr coefficients;
     const uint16_t* codes_ptr() const {
         return static_cast<const uint16_t*>(codes->ptr) + codes_offset;
     }

@@ -25,6 +25,7 @@
 #include <cstdlib>
 
 #include "../internal.hpp"
+#include "gather_mma.hpp"
 #include "gemm_simt.hpp"
 #include "gemm_tcgen05.hpp"
 #include "views.cuh"
@@ -980,7 +981,7 @@ bool wide_group_supported(const csdr_context* ctx, const csdr_segment* const* se
 
 WideDx launch_wide_project(csdr_context* ctx, const csdr_segment* const* segs, uint32_t n, XPlanesView x, uint32_t M,
                            float* dx_base, const Exchange* xch, const float* blk_base, const float* sums,
-                           const NormShares* shares) {
+                           const NormShares* shares, bool fp32_dx) {
     if (n == 0 || n > kGatherGroupMax) throw Error(CSDR_ERR_LIMIT, "matmul group holds 1 to 4 segments");
     WideDx w{};
     if (M <= 16u) {
@@ -990,6 +991,18 @@ WideDx launch_wide_project(csdr_context* ctx, const csdr_segment* const* segs, u
     w.stride = w.tile_mt ? w.tile_mt : M;
     size_t total_atoms = 0;
     for (uint32_t i = 0; i < n; ++i) total_atoms += segs[i]->g.n_atoms;
+    bool as_planes = !fp32_dx && M > 16u && !(xch && xch->ranks > 1u);
+    for (uint32_t i = 0; i < n; ++i) as_planes = as_planes && gather_mma_supported(ctx, segs[i], M);
+    if (as_planes) {
+        w.stride = (M + 7u) & ~7u;
+        __nv_bfloat16* at = static_cast<__nv_bfloat16*>(ctx->scratch_get(0, total_atoms * w.stride * 6u));
+        for (uint32_t i = 0; i < n; ++i) {
+            w.planes[i] = DxPlanes{at, w.stride};
+            at += 3u * static_cast<size_t>(segs[i]->g.n_atoms) * w.stride;
+        }
+        launch_dx_tma_group(ctx, segs, n, x, M, nullptr, w.stride, nullptr, nullptr, nullptr, false, shares, w.planes);
+        return w;
+    }
     w.floats = total_atoms * w.stride;
     w.base = dx_base ? dx_base
                      : static_cast<float*>(ctx->scratch_get(0, total_atoms * std::max<size_t>(w.stride, 16u) * 4u));
@@ -1051,7 +1064,8 @@ uint32_t launch_wide_gather(csdr_context* ctx, const csdr_segment* const* segs, 
     }
     for (uint32_t i = 0; i < n; ++i) {
         YView yv{outs[i].y, y_layout, segs[i]->g.rows, M, 0u, M, outs[i].bias};
-        launch_gather_wide(ctx, segs[i], w.dx[i], M, yv, outs[i].residual, ts);
+        if (w.planes[i].p) launch_gather_mma(ctx, segs[i], w.planes[i], M, yv, outs[i].residual, ts);
+        else launch_gather_wide(ctx, segs[i], w.dx[i], M, yv, outs[i].residual, ts);
     }
     return 0u;
 }
@@ -1125,6 +1139,11 @@ void launch_matmul_tcgen05(csdr_context* ctx, const csdr_segment* seg, const Mat
     const uint32_t kb_per_split = (n_kb + n_split - 1u) / n_split;
     n_split = (n_kb + kb_per_split - 1u) / kb_per_split;
 
+    if (M > 16u && g.n_stages <= 64u && dx_tma_supported(ctx, seg, a.batch) && gather_mma_supported(ctx, seg, M)) {
+        const WideOut out{a.y, a.bias, nullptr};
+        launch_matmul_wide_group(ctx, &seg, 1, make_x_planes(ctx, a.x, a.x_dtype, a.x_layout, M, g.cols), M, &out, a.y_layout);
+        return;
+    }
     const size_t dx_floats = static_cast<size_t>(g.n_atoms) * M;
     float* dx = static_cast<float*>(ctx->scratch_get(0, std::max<size_t>(dx_floats * 4u, static_cast<size_t>(g.n_atoms) * 64u)));
     const bool use_tma = dx_tma_supported(ctx, seg, a.batch);

@@ -46,16 +46,24 @@ struct XPlanesView {
 XPlanesView make_x_planes(csdr_context* ctx, const void* x, int x_dtype, int x_layout, uint32_t M, uint32_t cols);
 struct Exchange;
 struct NormShares;
+// Dx of one segment as three bf16 planes hi | mid | lo, each [n_atoms][stride], whose sum is the fp32
+// projection to 24 bits; stride is a multiple of eight tokens. What the gather on the tensor cores
+// reads (gather_mma.hpp).
+struct DxPlanes {
+    __nv_bfloat16* p = nullptr;
+    uint32_t stride = 0;
+};
 // One projection launch for up to four dictionaries over the same activations (q|k|v, gate|up).
 // With an exchange (tensor parallelism, at most 16 tokens) the finished rows go into every
 // rank's slot for this rank, at the offsets dx[i] - blk_base, `sums` (this rank's per-token sums
 // of squares, or null) ride along at offset 0, and the launch's last CTA raises the flags: the
 // projection and its share of the collective are one kernel. transposed (one dictionary, no
 // exchange): Dx leaves token-major, [token][atom] with dx_stride floats between token rows.
-// shares: see NextNorm.
+// shares: see NextNorm. planes (one per dictionary): Dx leaves as planes instead of floats.
 void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uint32_t n_seg, XPlanesView x, uint32_t M,
                          float* const* dx, uint32_t dx_stride, const Exchange* xch, const float* blk_base,
-                         const float* sums, bool transposed = false, const NormShares* shares = nullptr);
+                         const float* sums, bool transposed = false, const NormShares* shares = nullptr,
+                         const DxPlanes* planes = nullptr);
 
 // Up to four row-tile segments over the same activation planes: one projection launch and, for
 // a single token tile (M <= 16), one gather launch for the whole group. y = W x (+ bias)
@@ -99,6 +107,7 @@ struct WideDx {
     float* dx[4];
     size_t floats;
     uint32_t stride, tile_mt;
+    DxPlanes planes[4];      // set: Dx lies here (context scratch) and not at dx[]
 };
 // Exchange of partial projections between tensor-parallel ranks through peer memory (one
 // process per GPU, regions mapped into each other with CUDA IPC). Every rank owns a region of
@@ -121,10 +130,11 @@ struct Exchange {
     uint32_t* done = nullptr;      // this rank's count of finished CTAs of the projection kernel (device)
     int* status = nullptr;         // context status word: a wait that ran out is recorded here
 };
-// The two halves of launch_matmul_wide_group. dx_base == nullptr: context scratch.
+// The two halves of launch_matmul_wide_group. dx_base == nullptr: context scratch. fp32_dx: the caller
+// adds to Dx between the two halves, so it has to be floats at dx[].
 WideDx launch_wide_project(csdr_context* ctx, const csdr_segment* const* segs, uint32_t n, XPlanesView x, uint32_t M,
                            float* dx_base, const Exchange* xch = nullptr, const float* blk_base = nullptr,
-                           const float* sums = nullptr, const NormShares* shares = nullptr);
+                           const float* sums = nullptr, const NormShares* shares = nullptr, bool fp32_dx = false);
 // Returns the number of CTAs that left shares when `next` was given and rode on the gather (one
 // member, single token tile, token-major y); 0 leaves the next norm's first half to the caller.
 uint32_t launch_wide_gather(csdr_context* ctx, const csdr_segment* const* segs, uint32_t n, const WideDx& w, uint32_t M,

@@ -115,7 +115,8 @@ struct Params {
     float* dx_of[kMaxGroup];              // each member's Dx, [K_s][dx_stride]
     uint32_t M;             // tokens
     uint32_t dx_stride;     // floats between Dx rows (>= M); transposed: between token rows (>= atoms)
-    uint32_t transposed;    // Dx leaves token-major, [token][atom], instead of [atom][token]
+    __nv_bfloat16* planes_of[kMaxGroup];  // kPlanes: each member's planes hi | mid | lo
+    uint32_t plane_elems[kMaxGroup];      // elements between a member's planes
     uint32_t n_tile;        // MMA N: 16, 32, 64 or 128
     uint32_t tmem_cols;     // power of two >= max(32, n_tile)
     uint32_t n_kb;          // C / 64
@@ -157,7 +158,12 @@ __device__ __forceinline__ void stamp(const Params& p, int slot) {
     }
 }
 
+// How Dx leaves: floats [atom][token], floats [token][atom], or bf16 planes. Instances, because the
+// branches cost the short launches (8 and 64 tokens) 2 % where they were decided at run time.
+enum class DxForm { kFloats, kTokenMajor, kPlanes };
+
 // grid (atom tiles of every member, token tiles, column ranges); cluster (1, 1, column ranges)
+template <DxForm FORM>
 __global__ void __launch_bounds__(kThreads, 1)
 hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ CUtensorMap map_xhi,
                    const __grid_constant__ CUtensorMap map_xlo, const __grid_constant__ Params p) {
@@ -184,6 +190,7 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
     for (uint32_t i = 1; i < kMaxGroup; ++i)
         if (i < p.n_seg && blockIdx.x >= p.tile_begin[i]) seg = i;
     const uint32_t atom0 = (blockIdx.x - p.tile_begin[seg]) * kTileM;
+    constexpr bool transposed = FORM == DxForm::kTokenMajor;
     float* const dx = p.dx_of[seg];
     const CUtensorMap* map_ahi = &maps.hi[seg];
     const CUtensorMap* map_alo = &maps.lo[seg];
@@ -364,7 +371,7 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
     const size_t xslot = (static_cast<size_t>(xseq & 1u) * p.xch_ranks + p.xch_rank) * p.xch_blk;
     // a finished piece of Dx: four tokens of one atom, to the local buffer or to every rank
     auto emit = [&](uint32_t atom, uint32_t tok, const float4& v, bool vec) {
-        if (p.transposed) {   // local only: four tokens of one atom go to four token rows
+        if (transposed) {   // local only: four tokens of one atom go to four token rows
             float* dst = dx + static_cast<size_t>(tok) * p.dx_stride + atom;
             dst[0] = v.x;
             if (tok + 1u < p.M) dst[p.dx_stride] = v.y;
@@ -373,6 +380,20 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
             return;
         }
         const size_t o = static_cast<size_t>(atom) * p.dx_stride + tok;
+        if constexpr (FORM == DxForm::kPlanes) {   // four tokens always: the rows are padded to whole eights
+            const __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x, v.y), h1 = __floats2bfloat162_rn(v.z, v.w);
+            const float r0 = v.x - __low2float(h0), r1 = v.y - __high2float(h0), r2 = v.z - __low2float(h1), r3 = v.w - __high2float(h1);
+            const __nv_bfloat162 m0 = __floats2bfloat162_rn(r0, r1), m1 = __floats2bfloat162_rn(r2, r3);
+            const __nv_bfloat162 l0 = __floats2bfloat162_rn(r0 - __low2float(m0), r1 - __high2float(m0));
+            const __nv_bfloat162 l1 = __floats2bfloat162_rn(r2 - __low2float(m1), r3 - __high2float(m1));
+            __nv_bfloat16* dst = p.planes_of[seg] + o;
+            *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+            dst += p.plane_elems[seg];
+            *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&m0), *reinterpret_cast<const uint32_t*>(&m1));
+            dst += p.plane_elems[seg];
+            *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
+            return;
+        }
         if (p.xch_ranks > 1u) {
             const size_t xo = xslot + p.xch_off[seg] + o;
 #pragma unroll
@@ -404,7 +425,7 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
         // one rank and an aligned token count: the tile is Dx itself; otherwise this rank's slab
         const bool direct = n_ranks == 1u && ((p.M | p.dx_stride) & 3u) == 0;
         const uint32_t n4 = N / 4u;
-        if (direct && p.transposed) {
+        if (direct && transposed) {
             // token-major out: four consecutive atoms of one token per store, so that a warp writes
             // whole lines of a token's row
             constexpr uint32_t r4n = kTileM / 4u;
@@ -441,8 +462,10 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
         const bool vec = ((p.M | p.dx_stride) & 3u) == 0;
         const float* tile_part = p.part + static_cast<size_t>(tile) * n_ranks * kTileM * N;
         // neighbouring threads take neighbouring pieces of what is contiguous on the way out
-        auto row_of = [&](uint32_t i) { return p.transposed ? i % rows_mine : i / n4; };
-        auto c4_of = [&](uint32_t i) { return p.transposed ? i / rows_mine : i % n4; };
+        auto place = [&](uint32_t i, uint32_t& row, uint32_t& c4) {
+            row = row_begin + (transposed ? i % rows_mine : i / n4);
+            c4 = transposed ? i / rows_mine : i % n4;
+        };
         // two items per pass, every rank's piece of both requested before the first add: the
         // loads are L2 round trips and must overlap
         for (uint32_t i0 = tid; i0 < rows_mine * n4; i0 += 2u * kThreads) {
@@ -451,7 +474,8 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
             for (uint32_t h = 0; h < 2u; ++h) {
                 const uint32_t i = i0 + h * kThreads;
                 if (i < rows_mine * n4) {
-                    const uint32_t row = row_begin + row_of(i), c4 = c4_of(i);
+                    uint32_t row, c4;
+                    place(i, row, c4);
                     const float* src = tile_part + static_cast<size_t>(row) * N + c4 * 4u;
 #pragma unroll
                     for (uint32_t r = 0; r < 16u; ++r)
@@ -463,7 +487,8 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
             for (uint32_t h = 0; h < 2u; ++h) {
                 const uint32_t i = i0 + h * kThreads;
                 if (i >= rows_mine * n4) break;
-                const uint32_t row = row_begin + row_of(i), c4 = c4_of(i);
+                uint32_t row, c4;
+                place(i, row, c4);
                 float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (uint32_t r = 0; r < 16u; ++r)
@@ -802,7 +827,7 @@ XPlanesView make_x_planes(csdr_context* ctx, const void* x, int x_dtype, int x_l
 
 void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uint32_t n_seg, XPlanesView x, uint32_t M,
                          float* const* dx, uint32_t dx_stride, const Exchange* xch, const float* blk_base,
-                         const float* sums, bool transposed, const NormShares* shares) {
+                         const float* sums, bool transposed, const NormShares* shares, const DxPlanes* planes) {
     using namespace tma_detail;
     if (transposed && ((xch && xch->ranks > 1u) || n_seg != 1u))
         throw Error(CSDR_ERR_INVALID_ARG, "a token-major projection is local and has one dictionary");
@@ -820,11 +845,15 @@ void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uin
     uint32_t atom_tiles = 0;
     for (uint32_t i = 0; i < n_seg; ++i) {
         if (segs[i]->g.cols != cols) throw Error(CSDR_ERR_GEOMETRY, "projection group: members differ in columns");
-        auto planes = planes_for(ctx, segs[i]);
-        maps.hi[i] = planes->map_hi;
-        maps.lo[i] = planes->map_lo;
+        auto weights = planes_for(ctx, segs[i]);
+        maps.hi[i] = weights->map_hi;
+        maps.lo[i] = weights->map_lo;
         p.tile_begin[i] = atom_tiles;
-        p.dx_of[i] = dx[i];
+        p.dx_of[i] = dx ? dx[i] : nullptr;
+        if (planes) {
+            p.planes_of[i] = planes[i].p;
+            p.plane_elems[i] = segs[i]->g.n_atoms * planes[i].stride;
+        }
         atom_tiles += segs[i]->g.n_atoms / kTileM;
     }
     for (uint32_t i = n_seg; i <= kMaxGroup; ++i) p.tile_begin[i] = atom_tiles;
@@ -835,11 +864,14 @@ void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uin
 
     const size_t smem_max = ctx->smem_optin - 4096u;   // static barriers, the shares block and alignment slack
     if (!ctx->tma_attrs_set) {
-        ctx->opt_in_smem(reinterpret_cast<const void*>(hsdr_dx_tma_kernel), smem_max);
-        if (cudaFuncSetAttribute(hsdr_dx_tma_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
-            ctx->tma_max_cluster = 16;
-        else
-            (void)cudaGetLastError();
+        ctx->tma_max_cluster = 16;
+        for (auto kern : {hsdr_dx_tma_kernel<DxForm::kFloats>, hsdr_dx_tma_kernel<DxForm::kTokenMajor>, hsdr_dx_tma_kernel<DxForm::kPlanes>}) {
+            ctx->opt_in_smem(reinterpret_cast<const void*>(kern), smem_max);
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+                (void)cudaGetLastError();
+                ctx->tma_max_cluster = 8;
+            }
+        }
         ctx->tma_attrs_set = true;
     }
     const int max_cluster = ctx->tma_max_cluster;
@@ -878,7 +910,7 @@ void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uin
             cfg.gridDim = dim3(atom_tiles, tok_tiles, r);
             attr[0].val.clusterDim.z = r;
             int n_clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&n_clusters, hsdr_dx_tma_kernel, &cfg) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&n_clusters, hsdr_dx_tma_kernel<DxForm::kFloats>, &cfg) != cudaSuccess) {
                 (void)cudaGetLastError();
                 n_clusters = 0;
             }
@@ -894,7 +926,6 @@ void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uin
 
     p.M = M;
     p.dx_stride = dx_stride;
-    p.transposed = transposed ? 1u : 0u;
     p.n_tile = N;
     p.tmem_cols = std::max(32u, N);
     p.n_kb = n_kb;
@@ -935,7 +966,8 @@ void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uin
         p.norm_sumsq = shares->sumsq;
     }
     LaunchScope ls(ctx, KC_GEMM);
-    CSDR_CUDA(cudaLaunchKernelEx(&cfg, hsdr_dx_tma_kernel, maps, map_xhi, map_xlo, p));
+    auto kern = transposed ? hsdr_dx_tma_kernel<DxForm::kTokenMajor> : planes ? hsdr_dx_tma_kernel<DxForm::kPlanes> : hsdr_dx_tma_kernel<DxForm::kFloats>;
+    CSDR_CUDA(cudaLaunchKernelEx(&cfg, kern, maps, map_xhi, map_xlo, p));
     ls.done("hsdr_dx_tma_kernel");
 }
 
