@@ -240,7 +240,9 @@ void launch_dense_matmul(csdr_context* ctx, const float* W_dev, uint32_t R, uint
                          const MatmulArgs& a, bool w_fresh);
 
 // Row tiles the tensor-core path refuses (fp32 projection on the CUDA cores, then the gathers).
-bool simt_rows_supported(const csdr_context* ctx, const csdr_segment* seg, size_t batch);
-void matmul_rows_simt(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs& a);
+// dictionary: elements of all dictionaries of the launch (0: of this one).
+bool simt_rows_supported(const csdr_context* ctx, const csdr_segment* seg, size_t batch, size_t dictionary = 0);
+// n products of one width, batch and form, each of its own segment and activations.
+void matmul_rows_simt(csdr_context* ctx, const csdr_segment* const* segs, const MatmulArgs* args, uint32_t n);
 
 }  // namespace csdr

@@ -37,11 +37,16 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 }
 
 struct SimtParams {
-    const float* W;
+    struct {
+        const float* W;
+        const void* x;
+        uint32_t rows, row_off, tile0;   // rows of the member, where they start in the result, its first row tile
+    } m[kSimtMembers];
+    uint32_t n_members;
     uint32_t rows, cols, n_kb, kb_per_split, n_split;
-    uint32_t vec;      // rows of W start on 16-byte boundaries
+    uint32_t vec;      // rows of every W start on 16-byte boundaries
     uint32_t w_fresh;  // W is the output of earlier work on the stream
-    XView x;
+    XView x;           // x.x: see m
     YView y;           // n_split == 1
     float* part;       // [split][rows][tokens] otherwise
 };
@@ -49,14 +54,16 @@ struct SimtParams {
 // A thread's share of the 64 x 32 blocks of W: where its copies come from and go to, fixed but for
 // the column. What lies outside the matrix becomes zero.
 struct WBlock {
+    const float* W;
     const float* src;      // of the first copy at column 0
     uint32_t dst, c, rows_in;
-    __device__ __forceinline__ WBlock(const SimtParams& p, uint32_t row0, uint32_t tid) {
+    __device__ __forceinline__ WBlock(const SimtParams& p, const float* w, uint32_t rows, uint32_t row0, uint32_t tid) {
+        W = w;
         const uint32_t r = p.vec ? tid >> 3 : tid >> 5;
         c = p.vec ? (tid & 7u) * 4u : tid & 31u;
-        src = p.W + static_cast<size_t>(row0 + r) * p.cols + c;
+        src = W + static_cast<size_t>(row0 + r) * p.cols + c;
         dst = (r * kPitch + c) * 4u;
-        rows_in = p.rows > row0 + r ? p.rows - row0 - r : 0u;     // rows of the matrix from this copy's on
+        rows_in = rows > row0 + r ? rows - row0 - r : 0u;         // rows of the matrix from this copy's on
     }
     __device__ __forceinline__ void load(const SimtParams& p, const float* ws, uint32_t c0) const {
         const uint32_t base = smem_u32(ws) + dst;
@@ -67,7 +74,7 @@ struct WBlock {
             for (uint32_t i = 0; i < kRows / step; ++i) {
                 const bool in = col && i * step < rows_in;
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + i * step * kPitch * 4u),
-                             "l"(in ? src + c0 + static_cast<size_t>(i) * step * p.cols : p.W), "r"(in ? 16u : 0u)
+                             "l"(in ? src + c0 + static_cast<size_t>(i) * step * p.cols : W), "r"(in ? 16u : 0u)
                              : "memory");
             }
         } else {
@@ -76,7 +83,7 @@ struct WBlock {
             for (uint32_t i = 0; i < kRows / step; ++i) {
                 const bool in = col && i * step < rows_in;
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(base + i * step * kPitch * 4u),
-                             "l"(in ? src + c0 + static_cast<size_t>(i) * step * p.cols : p.W), "r"(in ? 4u : 0u)
+                             "l"(in ? src + c0 + static_cast<size_t>(i) * step * p.cols : W), "r"(in ? 4u : 0u)
                              : "memory");
             }
         }
@@ -90,17 +97,19 @@ template <uint32_t TOK, typename X, bool FEATURE_MAJOR>
 struct XBlock {
     static constexpr uint32_t N = TOK * kCols / kThreads;
     static constexpr uint32_t step_t = FEATURE_MAJOR ? 0u : kThreads / kCols, step_c = FEATURE_MAJOR ? kThreads / TOK : 0u;
+    const X* x;
     const X* src;
     uint32_t t, c, toks_in;
     size_t stride;         // between this thread's elements; col: between neighbouring columns
     size_t col;
     float v[N];
-    __device__ __forceinline__ XBlock(const SimtParams& p, uint32_t t0, uint32_t tid) {
+    __device__ __forceinline__ XBlock(const SimtParams& p, const void* from, uint32_t t0, uint32_t tid) {
+        x = static_cast<const X*>(from);
         t = FEATURE_MAJOR ? tid % TOK : tid / kCols;
         c = FEATURE_MAJOR ? tid / TOK : tid % kCols;
         const size_t tok = FEATURE_MAJOR ? 1u : p.x.C;
         col = FEATURE_MAJOR ? p.x.Mtotal : 1u;
-        src = static_cast<const X*>(p.x.x) + (p.x.b0 + t0 + t) * tok + c * col;
+        src = x + (p.x.b0 + t0 + t) * tok + c * col;
         stride = step_t * tok + step_c * col;
         toks_in = p.x.M > t0 + t ? p.x.M - t0 - t : 0u;
     }
@@ -119,7 +128,7 @@ struct XBlock {
         for (uint32_t i = 0; i < N; ++i) {
             const bool in = i * step_t < toks_in && i * step_c < cols_in;
             asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(base + (i * step_t * kPitch + i * step_c) * 4u),
-                         "l"(in ? static_cast<const void*>(at + i * stride) : p.x.x), "r"(in ? 4u : 0u)
+                         "l"(in ? at + i * stride : x), "r"(in ? 4u : 0u)
                          : "memory");
         }
     }
@@ -145,15 +154,19 @@ hsdr_gemm_simt_kernel(const __grid_constant__ SimtParams p) {
     constexpr uint32_t TB = B >= 32u ? 16u : 8u, TA = kThreads / TB;     // threads along each
     constexpr uint32_t NA = A / TA, NB = B / TB;
     const uint32_t tid = threadIdx.x, tb = tid % TB, ta = tid / TB;
-    const uint32_t row0 = blockIdx.x * kRows, t0 = blockIdx.y * TOK;
+    uint32_t mi = 0;
+    for (uint32_t i = 1; i < p.n_members; ++i)
+        if (blockIdx.x >= p.m[i].tile0) mi = i;
+    const uint32_t rows = p.m[mi].rows, row_off = p.m[mi].row_off;
+    const uint32_t row0 = (blockIdx.x - p.m[mi].tile0) * kRows, t0 = blockIdx.y * TOK;
     const uint32_t kb0 = blockIdx.z * p.kb_per_split, kb1 = min(p.n_kb, kb0 + p.kb_per_split);
     unsigned long long acc[NA][NB];
 #pragma unroll
     for (uint32_t i = 0; i < NA; ++i)
 #pragma unroll
         for (uint32_t j = 0; j < NB; ++j) acc[i][j] = 0ull;
-    const WBlock wb(p, row0, tid);
-    XBlock<TOK, X, FEATURE_MAJOR> xb(p, t0, tid);
+    const WBlock wb(p, p.m[mi].W, rows, row0, tid);
+    XBlock<TOK, X, FEATURE_MAJOR> xb(p, p.m[mi].x, t0, tid);
     // a resident weight is no other launch's output; a rebuilt one and the activations may be
     if (p.w_fresh) asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
@@ -203,8 +216,8 @@ hsdr_gemm_simt_kernel(const __grid_constant__ SimtParams p) {
 #pragma unroll
         for (uint32_t j = 0; j < NB; ++j) {
             const uint32_t a = ta + i * TA, b = tb + j * TB;
-            const uint32_t r = row0 + (SWAP ? b : a), t = t0 + (SWAP ? a : b);
-            if (r >= p.rows || t >= p.x.M) continue;
+            const uint32_t in = row0 + (SWAP ? b : a), r = row_off + in, t = t0 + (SWAP ? a : b);
+            if (in >= rows || t >= p.x.M) continue;
             const float v = __uint_as_float(static_cast<uint32_t>(acc[i][j])) + __uint_as_float(static_cast<uint32_t>(acc[i][j] >> 32));
             if (p.n_split > 1u) {
                 const size_t o = SWAP ? static_cast<size_t>(t) * p.rows + r : static_cast<size_t>(r) * p.x.M + t;
@@ -241,17 +254,30 @@ simt_reduce_kernel(const float* __restrict__ part, uint32_t rows, uint32_t M, ui
 
 void launch_gemm_simt(csdr_context* ctx, const float* W, uint32_t rows, uint32_t cols, const XView& x, const YView& y,
                       bool w_fresh) {
+    const SimtMember one{W, x.x, rows, 0u};
+    launch_gemm_simt_many(ctx, &one, 1, rows, cols, x, y, w_fresh);
+}
+
+void launch_gemm_simt_many(csdr_context* ctx, const SimtMember* members, uint32_t n_members, uint32_t rows, uint32_t cols, const XView& x,
+                           const YView& y, bool w_fresh) {
     if (rows == 0 || x.M == 0) return;
+    if (n_members == 0 || n_members > kSimtMembers) throw Error(CSDR_ERR_LIMIT, "fp32 product: 1 to 16 members");
     const bool swap = y.layout == CSDR_LAYOUT_TOKEN_MAJOR;
     const uint32_t tok = x.M <= 16u ? 16u : x.M <= 32u ? 32u : 64u;
     SimtParams p{};
-    p.W = W;
     p.rows = rows;
     p.cols = cols;
-    p.vec = cols % 4u == 0 && (reinterpret_cast<uintptr_t>(W) & 15u) == 0;
+    p.vec = cols % 4u == 0;
+    p.n_members = n_members;
+    uint32_t row_tiles = 0;
+    for (uint32_t i = 0; i < n_members; ++i) {
+        p.m[i] = {members[i].W, members[i].x, members[i].rows, members[i].row_off, row_tiles};
+        p.vec = p.vec && (reinterpret_cast<uintptr_t>(members[i].W) & 15u) == 0;
+        row_tiles += (members[i].rows + kRows - 1u) / kRows;
+    }
     p.w_fresh = w_fresh ? 1u : 0u;
     p.n_kb = (cols + kCols - 1u) / kCols;
-    const uint32_t row_tiles = (rows + kRows - 1u) / kRows, tok_tiles = (x.M + tok - 1u) / tok;
+    const uint32_t tok_tiles = (x.M + tok - 1u) / tok;
     // column ranges: enough CTAs for four per SM, at least two blocks of columns each, and partial
     // sums that stay in L2
     const uint64_t tiles = static_cast<uint64_t>(row_tiles) * tok_tiles, want = 4ull * static_cast<uint32_t>(ctx->sm_count);

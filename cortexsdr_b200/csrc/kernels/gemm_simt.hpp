@@ -17,4 +17,15 @@ namespace csdr {
 void launch_gemm_simt(csdr_context* ctx, const float* W, uint32_t rows, uint32_t cols, const XView& x, const YView& y,
                       bool w_fresh);
 
+// The same for several weights of one width, each over its own activations (x.x is not read; the form of
+// all is x's): member i's rows start at row row_off of the result, which has `rows` rows in all.
+constexpr uint32_t kSimtMembers = 16;
+struct SimtMember {
+    const float* W;
+    const void* x;
+    uint32_t rows, row_off;
+};
+void launch_gemm_simt_many(csdr_context* ctx, const SimtMember* members, uint32_t n_members, uint32_t rows, uint32_t cols, const XView& x,
+                           const YView& y, bool w_fresh);
+
 }  // namespace csdr

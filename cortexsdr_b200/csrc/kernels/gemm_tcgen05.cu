@@ -1211,35 +1211,69 @@ void launch_matmul_tcgen05(csdr_context* ctx, const csdr_segment* seg, const Mat
 // of 1024: 10.4 against 9.2, 128 of 2048: 9.9 against 9.1; 300 of 512, below the line: 8.1 against
 // 13.4; up to four tokens 512 of 4096: 11.8 against 12.7), and past its sixteen tokens always. The
 // bounds are the gathers' shared memory.
-bool simt_rows_supported(const csdr_context* ctx, const csdr_segment* seg, size_t batch) {
+namespace {
+// Shared memory of a group gather over `rows` rows in all.
+size_t group_gather_smem(const csdr_context* ctx, uint64_t rows, uint32_t slots, uint32_t atoms) {
+    const uint64_t ctas = 2ull * static_cast<uint32_t>(ctx->sm_count), per = std::max<uint64_t>(kGroupThreads, (rows + ctas - 1u) / ctas);
+    return per * slots * 2u + static_cast<size_t>(atoms) * 64u + 1024u;
+}
+}  // namespace
+
+bool simt_rows_supported(const csdr_context* ctx, const csdr_segment* seg, size_t batch, size_t dictionary) {
     const Geometry& g = seg->g;
     if (!g.row_tiles() || batch > 0xFFFFFFFFull || g.slots() > kWideMaxSlots || g.n_stages > 64u) return false;
-    if (g.cols % 4u == 0 && (batch < ctx->simt_min_batch || (batch <= 16u && static_cast<size_t>(g.n_atoms) * g.cols < ctx->simt_min_dict)))
-        return false;
+    if (!dictionary) dictionary = static_cast<size_t>(g.n_atoms) * g.cols;
+    if (g.cols % 4u == 0 && (batch < ctx->simt_min_batch || (batch <= 16u && dictionary < ctx->simt_min_dict))) return false;
     if (batch > 16u) return gather_wide_smem(g.n_atoms) <= ctx->smem_optin;
-    const size_t rows_per_cta = std::max<size_t>(kGroupThreads, (g.rows + 2u * ctx->sm_count - 1u) / (2u * ctx->sm_count));
-    return rows_per_cta * g.slots() * 2u + static_cast<size_t>(g.n_atoms) * 64u + 1024u <= ctx->smem_optin;
+    return group_gather_smem(ctx, g.rows, g.slots(), g.n_atoms) <= ctx->smem_optin;
 }
 
-void matmul_rows_simt(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs& a) {
-    const Geometry& g = seg->g;
+void matmul_rows_simt(csdr_context* ctx, const csdr_segment* const* segs, const MatmulArgs* args, uint32_t n) {
+    const MatmulArgs& a = args[0];
     const uint32_t M = static_cast<uint32_t>(a.batch);
     uint32_t mt = M;
     if (M <= 16u)
         for (mt = 1; mt < M;) mt <<= 1;
-    float* dx = static_cast<float*>(ctx->scratch_get(0, static_cast<size_t>(g.n_atoms) * std::max(mt, 16u) * 4u));
-    launch_gemm_simt(ctx, static_cast<const float*>(seg->atoms->ptr), g.n_atoms, g.cols, XView{a.x, a.x_dtype, a.x_layout, g.cols, M, 0u, M},
-                     YView{dx, CSDR_LAYOUT_FEATURE_MAJOR, g.n_atoms, mt, 0u, M, nullptr}, false);
-    if (M <= 16u) {
-        WideDx w{};
-        w.base = w.dx[0] = dx;
-        w.floats = static_cast<size_t>(g.n_atoms) * mt;
-        w.stride = w.tile_mt = mt;
-        const WideOut out{a.y, a.bias, nullptr};
-        gather_tile_group(ctx, &seg, 1, w, M, &out, a.y_layout, TokenScale{});
-        return;
+    for (uint32_t i0 = 0; i0 < n; i0 += kSimtMembers) {
+        const uint32_t cnt = std::min(kSimtMembers, n - i0);
+        SimtMember m[kSimtMembers];
+        uint32_t rows = 0;
+        for (uint32_t i = 0; i < cnt; ++i) {
+            m[i] = SimtMember{static_cast<const float*>(segs[i0 + i]->atoms->ptr), args[i0 + i].x, segs[i0 + i]->g.n_atoms, rows};
+            rows += (segs[i0 + i]->g.n_atoms + 3u) & ~3u;     // every member's Dx starts on a 16-byte boundary
+        }
+        float* dx = static_cast<float*>(ctx->scratch_get(0, static_cast<size_t>(rows) * std::max(mt, 16u) * 4u));
+        launch_gemm_simt_many(ctx, m, cnt, rows, segs[0]->g.cols, XView{nullptr, a.x_dtype, a.x_layout, segs[0]->g.cols, M, 0u, M},
+                              YView{dx, CSDR_LAYOUT_FEATURE_MAJOR, rows, mt, 0u, M, nullptr}, false);
+        if (M > 16u) {
+            for (uint32_t i = 0; i < cnt; ++i) {
+                const MatmulArgs& b = args[i0 + i];
+                launch_gather_wide(ctx, segs[i0 + i], dx + static_cast<size_t>(m[i].row_off) * mt, M,
+                                   YView{b.y, b.y_layout, segs[i0 + i]->g.rows, M, 0u, M, b.bias}, nullptr, TokenScale{});
+            }
+            continue;
+        }
+        for (uint32_t j0 = 0, c; j0 < cnt; j0 += c) {
+            uint64_t rows_all = 0;
+            uint32_t slots = 0, atoms = 0;
+            for (c = 0; c < std::min(kGatherGroupMax, cnt - j0); ++c) {      // as many as one launch holds
+                const Geometry& g = segs[i0 + j0 + c]->g;
+                rows_all += g.rows;
+                slots = std::max(slots, g.slots());
+                atoms = std::max(atoms, g.n_atoms);
+                if (c && group_gather_smem(ctx, rows_all, slots, atoms) > ctx->smem_optin) break;
+            }
+            WideDx w{};
+            WideOut outs[kGatherGroupMax];
+            w.base = dx;
+            w.stride = w.tile_mt = mt;
+            for (uint32_t j = 0; j < c; ++j) {
+                w.dx[j] = dx + static_cast<size_t>(m[j0 + j].row_off) * mt;
+                outs[j] = WideOut{args[i0 + j0 + j].y, args[i0 + j0 + j].bias, nullptr};
+            }
+            gather_tile_group(ctx, segs + i0 + j0, c, w, M, outs, a.y_layout, TokenScale{});
+        }
     }
-    launch_gather_wide(ctx, seg, dx, M, YView{a.y, a.y_layout, g.rows, M, 0u, M, a.bias}, nullptr, TokenScale{});
 }
 
 }  // namespace csdr

@@ -749,7 +749,7 @@ void launch_matmul(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs&
         return;
     }
     if (simt_rows_supported(ctx, seg, a.batch)) {
-        matmul_rows_simt(ctx, seg, a);
+        matmul_rows_simt(ctx, &seg, &a, 1);
         return;
     }
     const bool fast_rows = g.row_tiles() && (g.cols % 4u == 0);

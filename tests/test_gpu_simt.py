@@ -54,3 +54,39 @@ def test_fp32_products(ctx, oracle, rows, cols, tile, atoms, k, m, dtype, token)
     got, xd = product(ctx, pay, x, dtype, token, bias)
     want = xd @ oracle.decompress(pay).astype(np.float64).T + bias
     assert np.linalg.norm(got - want) <= FP32 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("members,cols,m", [(3, 97, 3), (5, 97, 16), (2, 1024, 40), (18, 33, 1)])
+def test_groups_of_fp32_products(ctx, oracle, members, cols, m):
+    """One activation, members of 10 to 78 atoms (projections off 16-byte steps), more than a gather
+    launch or a projection launch holds."""
+    pays = [synth.hsdr_payload(50 + 7 * i, cols, n_atoms=10 + 4 * i + i % 3, k=3 + i % 4, seed=i) for i in range(members)]
+    segs = [cs.Segment.from_payload(p, ctx) for p in pays]
+    x = torch.from_numpy(np.random.default_rng(m).normal(0, 1, (m, cols)).astype(np.float32)).cuda()
+    ys = [torch.full((m, s.rows), float("nan"), device="cuda") for s in segs]
+    torch.cuda.synchronize()
+    cs.Segment.matmul_group_device(segs, x.data_ptr(), cs.DTYPE_F32, cs.TOKEN_MAJOR, m, [y.data_ptr() for y in ys], cs.TOKEN_MAJOR)
+    ctx.synchronize()
+    xd = x.double().cpu().numpy()
+    for pay, y in zip(pays, ys):
+        want = xd @ oracle.decompress(pay).astype(np.float64).T
+        assert np.linalg.norm(y.double().cpu().numpy() - want) <= FP32 * np.linalg.norm(want)
+
+
+def test_lists_of_odd_width(ctx, oracle):
+    """Independent products share launches; one that reads another's result comes behind it; a different
+    width or form starts anew."""
+    rng = np.random.default_rng(5)
+    shapes = [(31, 45), (64, 45), (45, 31), (77, 45), (20, 99), (33, 99)]     # the third reads the first's result
+    pays = [synth.hsdr_payload(r, c, n_atoms=20, k=4, seed=r + c) for r, c in shapes]
+    segs = [cs.Segment.from_payload(p, ctx) for p in pays]
+    xs = [torch.from_numpy(rng.normal(0, 1, (2, c)).astype(np.float32)).cuda() for _, c in shapes]
+    ys = [torch.full((2, r), float("nan"), device="cuda") for r, _ in shapes]
+    xs[2] = ys[0]
+    torch.cuda.synchronize()
+    cs.Segment.matmul_queue_device([(s, x.data_ptr(), cs.DTYPE_F32, cs.TOKEN_MAJOR, 2, y.data_ptr(), cs.TOKEN_MAJOR, 0, 0 if i == 2 else -1)
+                                    for i, (s, x, y) in enumerate(zip(segs, xs, ys))])
+    ctx.synchronize()
+    for pay, x, y in zip(pays, xs, ys):
+        want = x.double().cpu().numpy() @ oracle.decompress(pay).astype(np.float64).T
+        assert np.linalg.norm(y.double().cpu().numpy() - want) <= FP32 * np.linalg.norm(want)
