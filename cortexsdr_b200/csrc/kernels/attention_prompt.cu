@@ -3,14 +3,15 @@
 // repeat_kv_heads, api/cortex_sdk.cpp:1453-1478), fp32 scores, weights and sums.
 //
 // attention_kernel walks the cache once per (token, head), which is right for a decode step; for a
-// prompt of T tokens it reads every key T / 2 times through L2 (1024 tokens, 32 heads of 128: 772 us,
-// here 369).
+// prompt of T tokens it reads every key T / 2 times through L2 (1024 tokens, 32 heads of 128: 767 us,
+// here 263).
 // Here a CTA owns 64 query rows of one kv head - rows run over (token, query head of the group), so
 // grouped heads share the keys too - and takes 64 keys at a time through shared memory: scores as a
 // 64 x 64 tile (4 x 4 a thread, packed fp32 multiply-adds over pairs of columns), an online softmax
 // whose rows live in 16 neighbouring lanes, and the weighted sum of the values (4 rows x HD / 16
 // columns a thread). Keys and values of a step share one buffer, so two CTAs fit an SM and one loads
-// while the other computes. The bound is fp32 issue.
+// while the other computes. The bound is shared-memory bandwidth
+// (77 % of it while the SMs are busy) and fp32 issue.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -81,7 +82,8 @@ __device__ __forceinline__ void load_keys(const KV* src, size_t row, uint32_t n,
     }
 }
 
-// grid (row blocks, kv heads); the blocks with the most keys start first
+// grid (kv heads, row blocks): the row blocks with the most keys start first, of every head (with the
+// heads on the slow dimension a third of the SMs' time went into the tail: 369 us)
 template <typename KV, int HD>
 __global__ void __launch_bounds__(kAttnThreads, 2)
 attention_prompt_kernel(const float* __restrict__ q, const KV* __restrict__ kc, const KV* __restrict__ vc,
@@ -96,8 +98,8 @@ attention_prompt_kernel(const float* __restrict__ q, const KV* __restrict__ kc, 
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4;
-    const uint32_t rep = QH / KVH, rows = T * rep, kvh = blockIdx.y;
-    const uint32_t row0 = (gridDim.x - 1u - blockIdx.x) * kQ;
+    const uint32_t rep = QH / KVH, rows = T * rep, kvh = blockIdx.x;
+    const uint32_t row0 = (gridDim.y - 1u - blockIdx.y) * kQ;
     const int32_t p0 = pos_of[0];
     const size_t krow = static_cast<size_t>(KVH) * HD;
     const size_t base = static_cast<size_t>(seq_of[0]) * max_seq * krow + static_cast<size_t>(kvh) * HD;
@@ -242,7 +244,7 @@ void launch(csdr_context* ctx, const float* q, const void* kc, const void* vc, c
     const size_t smem = prompt_smem<HD>();
     ctx->opt_in_smem(reinterpret_cast<const void*>(kern), smem);
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((T * (QH / KVH) + kQ - 1u) / kQ, KVH, 1);
+    cfg.gridDim = dim3(KVH, (T * (QH / KVH) + kQ - 1u) / kQ, 1);
     cfg.blockDim = dim3(kAttnThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
@@ -270,8 +272,8 @@ void launch_kv(csdr_context* ctx, const float* q, const void* kc, const void* vc
 }  // namespace
 
 // Short prompts stay with the kernel that has a CTA for every (token, head): at 128 tokens it takes
-// 25 us against 29 (32 heads of 128) and 15 against 19 (14 heads of 64), at 256 64 against 47 and 28
-// against 29, at 512 214 against 137 and 80 against 50.
+// 25 us against 29 (32 heads of 128) and 15 against 19 (14 heads of 64), at 256 64 against 48 and 29
+// against 29, at 512 214 against 104 and 80 against 50.
 bool attention_prompt_supported(const csdr_context* ctx, uint32_t T, uint32_t HD) {
     return (HD == 64u || HD == 128u) && T >= ctx->prompt_attention_min;
 }
