@@ -759,15 +759,24 @@ void launch_matmul(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs&
                              a.batch * g.n_col_tiles * g.n_atoms * static_cast<size_t>(g.tile_rows) * 4u <= (1ull << 30);
     // 2-D tiles whose shape the tensor maps do not take (ragged edges, rows not in 128s): the rebuilt
     // weight stays with the segment as fp32 (4 bytes an element, as the planes above) and the product
-    // is a plain fp32 one. The factored form moves batch * (n_atoms * tile_rows + rows * slots) words
-    // of tile products per column tile where the weight has rows * tile_cols: taken where that is
-    // more, and from 16 tokens on; a weight below a megabyte is bound by launches either way and
-    // keeps the factored form, which needs no copy of it.
-    if (!g.row_tiles() && ctx->cache_2d && !planes_2d &&
-        (a.batch >= 16 ||
-         (a.batch * (static_cast<size_t>(g.n_atoms) * g.tile_rows + static_cast<size_t>(g.rows) * g.slots()) >=
-              static_cast<size_t>(g.rows) * g.tile_cols &&
-          (!factored_tc || static_cast<size_t>(g.rows) * g.cols >= (1u << 18))))) {
+    // is a plain fp32 one, from 16 tokens on and below that by what the factored form would cost.
+    // On the tensor cores it moves batch * (n_atoms * tile_rows + rows * slots) words of tile products
+    // per column tile where the weight has rows * tile_cols: left where that is more; a weight below a
+    // megabyte is bound by launches either way and keeps the form that needs no copy of it. On the CUDA
+    // cores its n_atoms * tile_rows * cols products a token run at an eighth of the rate at which the
+    // dense product takes in weights (factored against dense, 300 atoms of 128 x 128, 7636 x 3719: one
+    // token, 5 words a row, 49 / 59 us, two 88 / 60, six 232 / 60), and its three launches cost more
+    // than a weight of 16 MB that stays in L2 (3000 x 1000 in 16 x 16 tiles at one token 27 / 11).
+    const size_t tile_words = static_cast<size_t>(g.n_atoms) * g.tile_rows;
+    const bool dense_2d = a.batch >= 16 ||
+                          (factored_tc ? a.batch * (tile_words + static_cast<size_t>(g.rows) * g.slots()) >=
+                                                 static_cast<size_t>(g.rows) * g.tile_cols &&
+                                             static_cast<size_t>(g.rows) * g.cols >= (1u << 18)
+                                       : static_cast<size_t>(g.rows) * g.cols <= (1u << 22) ||
+                                             a.batch * tile_words >= 8u * static_cast<size_t>(g.rows) ||
+                                             a.batch * (tile_words + static_cast<size_t>(g.rows) * g.slots()) >=
+                                                 static_cast<size_t>(g.rows) * g.tile_cols);
+    if (!g.row_tiles() && ctx->cache_2d && !planes_2d && dense_2d) {
         if (!seg->dense) {
             auto dn = std::make_shared<csdr_segment>();
             dn->ctx = ctx;
