@@ -49,31 +49,58 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// K-major operand, 128-byte swizzle: 8 rows x 128 B per swizzle atom, atoms 1024 B apart.
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
-    d |= static_cast<uint64_t>(1) << 16;
-    d |= static_cast<uint64_t>(1024u >> 4) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(2) << 61;
-    return d;
-}
+// Descriptor of a K-major operand, 128-byte swizzle (8 rows x 128 B per swizzle atom, atoms 1024 B
+// apart): the half that holds the address, in 16-byte units so that offsets add, and the other one.
+__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
 
 // kind::f16: D fp32, A and B bf16, both K-major, M = 128, N = n.
 __device__ __forceinline__ uint32_t make_idesc(uint32_t n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((kTileM >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
+// One lane issues while its warp goes along: what the products are made of stays uniform, and the
+// issue of a 64-column block - which bounds the whole kernel where the products are small - is a
+// straight line of additions (with descriptors put together for every product and the ring's places
+// divided out, a block took 0.5 us, whatever its size).
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate,
+                                         uint32_t leader) {
     asm volatile(
         "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        ".reg .pred p, q;\n"
+        ".reg .b64 a, b;\n"
+        "setp.ne.b32 p, %5, 0;\n"
+        "setp.ne.b32 q, %6, 0;\n"
+        "mov.b64 a, {%1, %4};\n"
+        "mov.b64 b, {%2, %4};\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n"
         "}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHi), "r"(accumulate), "r"(leader)
+        : "memory");
+}
+
+// The products of one 64-column block: hi*hi + lo*hi [+ hi*lo], four steps of 16 columns 32 bytes
+// apart. a, b: descriptors of the hi operands; lo_a, lo_b: from there to the lo ones.
+template <bool X_LO>
+__device__ __forceinline__ void mma_block(uint32_t d_tmem, uint32_t a, uint32_t lo_a, uint32_t b, uint32_t lo_b, uint32_t idesc,
+                                          uint32_t first, uint32_t leader) {
+#pragma unroll
+    for (uint32_t k = 0; k < kBlockK / 16u; ++k) {
+        mma_bf16(d_tmem, a + 2u * k, b + 2u * k, idesc, k ? 1u : first ^ 1u, leader);
+        mma_bf16(d_tmem, a + lo_a + 2u * k, b + 2u * k, idesc, 1u, leader);
+        if (X_LO) mma_bf16(d_tmem, a + 2u * k, b + lo_b + 2u * k, idesc, 1u, leader);
+    }
+}
+
+// Arrives on the barrier once every product issued so far has been done.
+__device__ __forceinline__ void mma_commit(uint32_t bar, uint32_t leader) {
+    asm volatile(
+        "{\n"
+        ".reg .pred q;\n"
+        "setp.ne.b32 q, %1, 0;\n"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+        "}\n" ::"r"(bar),
+        "r"(leader)
         : "memory");
 }
 
@@ -243,9 +270,9 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
                 tma_load_2d(dst + 2u * kATile, &map_xhi, c0, tok0, bar);
                 if (p.x_has_lo) tma_load_2d(dst + 2u * kATile + b_tile, &map_xlo, c0, tok0, bar);
             }
+            uint32_t s = 0, parity = 0;        // pre == p.stages here: the ring starts over
             for (uint32_t it = pre; it < n_it; ++it) {
-                const uint32_t s = it % p.stages, use = it / p.stages;
-                if (!mbar_wait(smem_u32(&empty_bar[s]), (use - 1u) & 1u, p.spin)) {
+                if (!mbar_wait(smem_u32(&empty_bar[s]), parity, p.spin)) {
                     failed_s = 1;
                     break;
                 }
@@ -259,41 +286,38 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
                 tma_load_2d(dst + kATile, map_alo, c0, atom0, bar);
                 tma_load_2d(dst + 2u * kATile, &map_xhi, c0, tok0, bar);
                 if (p.x_has_lo) tma_load_2d(dst + 2u * kATile + b_tile, &map_xlo, c0, tok0, bar);
+                if (++s == p.stages) {
+                    s = 0;
+                    parity ^= 1u;
+                }
             }
         }
     } else if (warp == 1) {
         // ---- MMA issue ----
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc(N);
-            for (uint32_t it = 0; it < n_it; ++it) {
-                const uint32_t s = it % p.stages, use = it / p.stages;
-                if (!mbar_wait(smem_u32(&full_bar[s]), use & 1u, p.spin)) {
-                    failed_s = 1;
-                    break;
-                }
-                if (failed_s) break;
-                if (it == 0) stamp(p, 2);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a_hi = smem_u32(smem + s * stage_bytes), a_lo = a_hi + kATile;
-                const uint32_t b_hi = a_hi + 2u * kATile, b_lo = b_hi + b_tile;
-#pragma unroll
-                for (uint32_t k = 0; k < kBlockK / 16u; ++k) {     // four K = 16 steps, 32 bytes apart
-                    const uint64_t ah = make_desc(a_hi + k * 32u), al = make_desc(a_lo + k * 32u);
-                    const uint64_t bh = make_desc(b_hi + k * 32u);
-                    mma_bf16(tmem_base, ah, bh, idesc, (it | k) != 0u);
-                    mma_bf16(tmem_base, al, bh, idesc, 1u);
-                    if (p.x_has_lo) mma_bf16(tmem_base, ah, make_desc(b_lo + k * 32u), idesc, 1u);
-                }
-                // the stage is free again once every MMA issued so far has read it
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 smem_u32(&empty_bar[s]))
-                             : "memory");
+        const uint32_t idesc = make_idesc(N), leader = lane == 0u ? 1u : 0u;
+        const uint32_t ring = desc_lo(smem_u32(smem)), stage_step = stage_bytes >> 4;
+        const bool x_lo = p.x_has_lo != 0u;
+        uint32_t s = 0, parity = 0, at = ring;
+        for (uint32_t it = 0; it < n_it; ++it) {
+            const bool ok = mbar_wait(smem_u32(&full_bar[s]), parity, p.spin) && !failed_s;
+            if (!__all_sync(0xFFFFFFFFu, ok)) {
+                failed_s = 1;
+                break;
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&accum_bar))
-                         : "memory");
-            stamp(p, 3);
+            if (it == 0 && leader) stamp(p, 2);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (x_lo) mma_block<true>(tmem_base, at, kATile >> 4, at + (2u * kATile >> 4), b_tile >> 4, idesc, it == 0u, leader);
+            else mma_block<false>(tmem_base, at, kATile >> 4, at + (2u * kATile >> 4), b_tile >> 4, idesc, it == 0u, leader);
+            mma_commit(smem_u32(&empty_bar[s]), leader);   // the stage is free again once they have read it
+            at += stage_step;
+            if (++s == p.stages) {
+                s = 0;
+                parity ^= 1u;
+                at = ring;
+            }
         }
+        mma_commit(smem_u32(&accum_bar), leader);
+        if (leader) stamp(p, 3);
     }
     // ---- column-range reduction through L2. Every CTA writes its accumulator tile to the
     // launch's partial buffer, the cluster meets at its barrier (release/acquire at cluster scope
@@ -594,16 +618,22 @@ hsdr_tile_project_mma_kernel(const __grid_constant__ CUtensorMap map_hi, const _
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     __syncthreads();
-    auto load = [&](uint32_t it) {      // weight block it of this CTA's walk: nobody else's output, read ahead
-        const uint32_t s = it % p.stages, tile = blockIdx.x + it / p.n_kb * gridDim.x, kb = it % p.n_kb;
-        const uint32_t bar = smem_u32(&full_bar[s]), dst = smem_u32(ring + s * stage_bytes);
+    // weight blocks of this CTA's walk, nobody else's output: read ahead
+    uint32_t l_stage = 0, l_tile = blockIdx.x, l_kb = 0;
+    auto load = [&]() {
+        const uint32_t bar = smem_u32(&full_bar[l_stage]), dst = smem_u32(ring + l_stage * stage_bytes);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(stage_bytes) : "memory");
-        tma_load_2d(dst, &map_hi, kb * kBlockK, tile * kTileM, bar);
-        tma_load_2d(dst + kATile, &map_lo, kb * kBlockK, tile * kTileM, bar);
+        tma_load_2d(dst, &map_hi, l_kb * kBlockK, l_tile * kTileM, bar);
+        tma_load_2d(dst + kATile, &map_lo, l_kb * kBlockK, l_tile * kTileM, bar);
+        if (++l_stage == p.stages) l_stage = 0;
+        if (++l_kb == p.n_kb) {
+            l_kb = 0;
+            l_tile += gridDim.x;
+        }
     };
     const uint32_t pre = min(p.stages, n_it);
     if (tid == 0)
-        for (uint32_t it = 0; it < pre; ++it) load(it);
+        for (uint32_t it = 0; it < pre; ++it) load();
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // activations: eight columns of one (token, column tile) at a time, one 16-byte unit of the
     // 128-byte swizzled rows; columns past the tile and tokens past the end are zero
@@ -631,45 +661,42 @@ hsdr_tile_project_mma_kernel(const __grid_constant__ CUtensorMap map_hi, const _
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
     if (warp == 0) {
-        if (lane == 0)
-            for (uint32_t it = pre; it < n_it; ++it) {
-                if (!mbar_wait(smem_u32(&empty_bar[it % p.stages]), (it / p.stages - 1u) & 1u, p.spin)) failed_s = 1;
-                if (failed_s) break;
-                load(it);
-            }
-    } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = make_idesc(N);
-            bool ok = true;
-            for (uint32_t ti = 0; ti < mine && ok; ++ti) {
-                const uint32_t acc = ti & 1u, d = tmem_base + acc * N;
-                if (ti >= 2u) ok = mbar_wait(smem_u32(&acc_empty[acc]), (ti / 2u - 1u) & 1u, p.spin);
-                for (uint32_t kb = 0; kb < p.n_kb && ok; ++kb) {
-                    const uint32_t it = ti * p.n_kb + kb, s = it % p.stages;
-                    ok = mbar_wait(smem_u32(&full_bar[s]), (it / p.stages) & 1u, p.spin) && !failed_s;
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_hi = smem_u32(ring + s * stage_bytes), a_lo = a_hi + kATile;
-                    const uint32_t b_hi = smem_u32(xs + kb * x_planes * b_tile), b_lo = b_hi + b_tile;
-#pragma unroll
-                    for (uint32_t k = 0; k < kBlockK / 16u; ++k) {
-                        const uint64_t ah = make_desc(a_hi + k * 32u), al = make_desc(a_lo + k * 32u);
-                        const uint64_t bh = make_desc(b_hi + k * 32u);
-                        mma_bf16(d, ah, bh, idesc, (kb | k) != 0u);
-                        mma_bf16(d, al, bh, idesc, 1u);
-                        if (p.x_has_lo) mma_bf16(d, ah, make_desc(b_lo + k * 32u), idesc, 1u);
-                    }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                     smem_u32(&empty_bar[s]))
-                                 : "memory");
-                }
-                if (ok)
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                     smem_u32(&acc_full[acc]))
-                                 : "memory");
+            uint32_t parity = 0;               // pre == p.stages here: the ring starts over
+            for (uint32_t it = pre; it < n_it; ++it) {
+                if (!mbar_wait(smem_u32(&empty_bar[l_stage]), parity, p.spin)) failed_s = 1;
+                if (failed_s) break;
+                if (l_stage + 1u == p.stages) parity ^= 1u;
+                load();
             }
-            if (!ok) failed_s = 1;
         }
+    } else if (warp == 1) {
+        const uint32_t idesc = make_idesc(N), leader = lane == 0u ? 1u : 0u;
+        const uint32_t ring_lo = desc_lo(smem_u32(ring)), x_lo = desc_lo(smem_u32(xs)), stage_step = stage_bytes >> 4;
+        bool ok = true;
+        uint32_t s = 0, parity = 0, at = ring_lo;
+        for (uint32_t ti = 0; ti < mine && ok; ++ti) {
+            const uint32_t acc = ti & 1u, d = tmem_base + acc * N;
+            if (ti >= 2u) ok = mbar_wait(smem_u32(&acc_empty[acc]), (ti / 2u - 1u) & 1u, p.spin);
+            for (uint32_t kb = 0; kb < p.n_kb && ok; ++kb) {
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&full_bar[s]), parity, p.spin) && !failed_s);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t b = x_lo + kb * (x_planes * b_tile >> 4);
+                if (x_planes == 2u) mma_block<true>(d, at, kATile >> 4, b, b_tile >> 4, idesc, kb == 0u, leader);
+                else mma_block<false>(d, at, kATile >> 4, b, b_tile >> 4, idesc, kb == 0u, leader);
+                mma_commit(smem_u32(&empty_bar[s]), leader);
+                at += stage_step;
+                if (++s == p.stages) {
+                    s = 0;
+                    parity ^= 1u;
+                    at = ring_lo;
+                }
+            }
+            ok = __all_sync(0xFFFFFFFFu, ok);
+            if (ok) mma_commit(smem_u32(&acc_full[acc]), leader);
+        }
+        if (!ok) failed_s = 1;
     } else {
         const uint32_t quad = warp & 3u, row = quad * 32u + lane;
         for (uint32_t ti = 0; ti < mine; ++ti) {
