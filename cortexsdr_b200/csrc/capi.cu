@@ -158,6 +158,18 @@ void* csdr_context::scratch_get(int slot, size_t bytes) {
     return scratch[slot]->ptr;
 }
 
+void csdr_context::scratch_trim(int slot, size_t most) {
+    if (!scratch[slot] || scratch[slot]->bytes <= most) return;
+    CSDR_CUDA(cudaStreamSynchronize(stream));
+    scratch[slot].reset();
+}
+
+bool csdr_context::capturing() const {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    CSDR_CUDA(cudaStreamIsCapturing(stream, &status));
+    return status != cudaStreamCaptureStatusNone;
+}
+
 namespace csdr_hostio {
 
 // Host-buffer calls on small operands avoid the copy engines and the driver's stream wait:

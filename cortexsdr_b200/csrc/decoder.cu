@@ -611,6 +611,12 @@ void run_logits(csdr_decoder* d, uint32_t T, uint32_t t0, uint32_t n) {
     }
 }
 
+// To the host behind the work on the stream; the caller waits for the stream.
+void copy_out(csdr_context* ctx, void* dst, const void* src, size_t bytes) {
+    if (bytes >= HostCopier::kSmall) ctx->copies().download(dst, src, bytes);
+    else CSDR_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+}
+
 void need(csdr_decoder* d) {
     if (!d) throw Error(CSDR_ERR_INVALID_ARG, "decoder is null");
     require_ctx(d->ctx);
@@ -976,7 +982,7 @@ int csdr_decoder_forward(csdr_decoder* d, uint32_t seq, const int32_t* tokens, s
             CSDR_CUDA(cudaMemcpyAsync(logits_out, d->logits->ptr, static_cast<size_t>(c.vocab) * 4,
                                       cudaMemcpyDeviceToHost, ctx->stream));
         }
-        if (hidden_out) ctx->copies().download(hidden_out, d->normed->ptr, static_cast<size_t>(T) * c.hidden * 4);
+        if (hidden_out) copy_out(ctx, hidden_out, d->normed->ptr, static_cast<size_t>(T) * c.hidden * 4);
         d->pos_host[seq] = p0 + static_cast<int32_t>(T);
         CSDR_CUDA(cudaMemcpyAsync(I32(d->pos_dev) + seq, &d->pos_host[seq], 4, cudaMemcpyHostToDevice, ctx->stream));
         CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1023,7 +1029,7 @@ int csdr_decoder_step(csdr_decoder* d, const int32_t* tokens, size_t batch, int3
         rethrow_last(csdr_decoder_step_device_async(d, I32(d->tokens_dev), batch, I32(d->next_dev)));
         CSDR_CUDA(cudaMemcpyAsync(next_out, d->next_dev->ptr, batch * 4, cudaMemcpyDeviceToHost, ctx->stream));
         if (logits_out)
-            ctx->copies().download(logits_out, d->logits->ptr, batch * d->cfg.vocab * 4);
+            copy_out(ctx, logits_out, d->logits->ptr, batch * d->cfg.vocab * 4);
         CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
     });
 }

@@ -223,6 +223,8 @@ int csdr_hsdr_encode(csdr_context* ctx, const float* W, uint32_t rows, uint32_t 
         uint8_t* codes_at = dict_at + 4u * static_cast<size_t>(n_atoms) * T;
         ctx->copies().download(dict_at, D->ptr, 4u * static_cast<size_t>(n_atoms) * T);
         ctx->copies().download(codes_at, codes, n_codes * 2);
+        // what an uncommonly large tensor needed is not kept for the next call
+        for (int slot : {2, 7, 8, 9, 10}) ctx->scratch_trim(slot, 256u << 20);
         // raw strips: top-right, then bottom (:1185-1197)
         uint8_t* e = codes_at + 2u * n_codes;
         const size_t wr = static_cast<size_t>(cols - C_full) * 4;

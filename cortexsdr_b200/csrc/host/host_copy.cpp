@@ -10,7 +10,6 @@ namespace csdr {
 
 namespace {
 constexpr size_t kSlot = 512u << 10;      // bytes of a page-locked slot
-constexpr size_t kSmall = 4u << 20;       // below: one copy by the driver (2 MB of logits took as long with the threads)
 constexpr size_t kMaxWorkers = 8;
 
 bool page_locked(const void* p) {

@@ -26,6 +26,8 @@ public:
     // Behind earlier work on the stream. On return the source of an upload may be reused; a download
     // is complete. Throws Error.
     void upload(void* dst, const void* src, size_t bytes) { copy(dst, src, bytes, true); }
+    // Below this many bytes a copy is the driver's (2 MB of logits took as long with the threads).
+    static constexpr size_t kSmall = 4u << 20;
     void download(void* dst, const void* src, size_t bytes) { copy(dst, src, bytes, false); }
 
 private:

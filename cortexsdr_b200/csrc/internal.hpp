@@ -108,6 +108,8 @@ struct csdr_context {
     }
     csdr::DevPtr scratch[11];  // 0 Dx, 1 tile products, 2 materialised W, 3 host staging, 4 fused-GEMV partials, 5 activation planes / wait self-test, 6 GEMV queue, 7 dense product before re-tiling, 8 - 10 encoder (dictionary, codes and small arrays, projections)
     void* scratch_get(int slot, size_t bytes);
+    void scratch_trim(int slot, size_t most);   // gives a slot back that has grown past `most` bytes
+    bool capturing() const;                     // the stream is being captured: nothing may be built on first use
     int* status_word = nullptr;  // device int: kernels record bounded-wait timeouts here
     // Page-locked, device-mapped host staging for the host-buffer entry points (grow-only).
     void* pinned = nullptr;
@@ -177,6 +179,8 @@ struct csdr_segment {
     // output row) whose cached bf16 planes feed the tensor-core kernel at wide batches - what the
     // reference's layer cache holds as fp32 after decompress(). Built on the first wide product.
     mutable std::shared_ptr<csdr_segment> dense;
+    // The same as fp32, for the shapes the tensor maps do not take.
+    mutable csdr::DevPtr dense_f32;
     // 2-D tile images only: the dictionary seen as n_atoms * tile_rows rows of tile_cols columns,
     // the shape in which the tensor-core projection computes all tile products of a few tokens.
     mutable std::shared_ptr<csdr_segment> tile_view;

@@ -493,7 +493,8 @@ bool gather_mma_supported(const csdr_context* ctx, const csdr_segment* seg, size
                             : g.n_atoms <= 256u ? batch <= kTok : batch <= 2u * kTok || pairs < 64u)
         return false;
     if (static_cast<uint64_t>((g.rows + kRowsTile - 1u) / kRowsTile) * kRowsTile * g.slots() > 0x7FFFFFFFull) return false;
-    return gather_mma_smem(g.n_atoms) + 1024u <= ctx->smem_optin && exact_in_bf16(seg->scales_host, g.k);
+    if (gather_mma_smem(g.n_atoms) + 1024u > ctx->smem_optin || !exact_in_bf16(seg->scales_host, g.k)) return false;
+    return seg->coefficients || !ctx->capturing();   // the entries are built on first use
 }
 
 void launch_gather_mma(csdr_context* ctx, const csdr_segment* seg, const DxPlanes& dx, uint32_t M, const YView& y, const float* residual,

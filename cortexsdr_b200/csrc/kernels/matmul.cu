@@ -10,7 +10,6 @@
 //                           decompress (:1340-1440) followed by the dense product of
 //                           SDRInferenceEngine::matmulForLayer (SparseInferenceEngine.cpp:1301-1310),
 //                           computed in factored form so the weight never exists in memory
-//   dense_rows_kernel       the same dense product for stored-raw fp32 segments
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -776,16 +775,15 @@ void launch_matmul(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs&
                                              a.batch * tile_words >= 8u * static_cast<size_t>(g.rows) ||
                                              a.batch * (tile_words + static_cast<size_t>(g.rows) * g.slots()) >=
                                                  static_cast<size_t>(g.rows) * g.tile_cols);
-    if (!g.row_tiles() && ctx->cache_2d && !planes_2d && dense_2d) {
-        if (!seg->dense) {
-            auto dn = std::make_shared<csdr_segment>();
-            dn->ctx = ctx;
-            dn->atoms = std::make_shared<DeviceBuffer>(static_cast<size_t>(g.rows) * g.cols * 4u, ctx->device);
-            launch_decode_rows(ctx, seg, nullptr, g.rows, static_cast<float*>(dn->atoms->ptr));
+    // (the rebuilt weight is made on first use: not while the stream is captured)
+    if (!g.row_tiles() && ctx->cache_2d && !planes_2d && dense_2d && (seg->dense_f32 || !ctx->capturing())) {
+        if (!seg->dense_f32) {
+            auto w = std::make_shared<DeviceBuffer>(static_cast<size_t>(g.rows) * g.cols * 4u, ctx->device);
+            launch_decode_rows(ctx, seg, nullptr, g.rows, static_cast<float*>(w->ptr));
             CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
-            seg->dense = dn;
+            seg->dense_f32 = w;
         }
-        launch_dense_matmul(ctx, static_cast<const float*>(seg->dense->atoms->ptr), g.rows, g.cols, a, false);
+        launch_dense_matmul(ctx, static_cast<const float*>(seg->dense_f32->ptr), g.rows, g.cols, a, false);
         return;
     }
     const size_t budget = std::min<size_t>(ctx->smem_optin, 200u * 1024u);
