@@ -489,8 +489,11 @@ void launch_t(csdr_context* ctx, FusedParams& p, uint32_t max_k, bool pdl) {
     // smallest grid this kernel can get (one CTA per SM), then launch with what fits.
     uint32_t all_k = 0;
     for (uint32_t i = 0; i < p.n_seg; ++i) all_k += p.seg[i].K;
-    // side by side as long as the slices leave room for two CTAs on an SM
-    const bool together = static_cast<size_t>(all_k) * (MT < 4 ? MT : 4) * 4u <= 32u * 1024u;
+    // Side by side as long as the slices leave room for two CTAs on an SM, and only where every CTA has at
+    // most one projection task: where they have more, the rows of one member are walked while the next
+    // one's projection is still under way (two 11008 x 4096: 10 to 11 us one after the other, 13 together).
+    const bool together = static_cast<size_t>(all_k) * (MT < 4 ? MT : 4) * 4u <= 32u * 1024u &&
+                          p.n_tasks <= 2u * static_cast<uint32_t>(ctx->sm_count);
     const uint32_t dx_atoms = together ? all_k : max_k;
     plan.dxs_segs = together ? p.n_seg : 1u;
     for (uint32_t i = 0; i < kMaxFusedGroup; ++i) plan.k_off[i + 1] = plan.k_off[i] + (i < p.n_seg ? p.seg[i].K : 0u);
