@@ -139,7 +139,8 @@ cudaError_t HostCopier::work_down(Worker& w) {
 void HostCopier::copy(void* dst, const void* src, size_t bytes, bool up) {
     if (!bytes) return;
     std::lock_guard<std::mutex> call(call_);
-    if (bytes < kSmall || page_locked(up ? src : dst) || !start()) {
+    // cudaStreamPerThread names another stream in every helper: its copies stay with the calling thread
+    if (bytes < kSmall || stream_ == cudaStreamPerThread || page_locked(up ? src : dst) || !start()) {
         CSDR_CUDA(cudaMemcpyAsync(dst, src, bytes, up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, stream_));
         // a page-locked source is read behind the call's return: wait, as for a download
         CSDR_CUDA(cudaStreamSynchronize(stream_));
