@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "internal.hpp"
+#include "kernels/gemm_simt.hpp"
 #include "kernels/gemm_tcgen05.hpp"
 #include "kernels/gemv_fused.hpp"
 #include "kernels/gemv_queue.hpp"
@@ -106,17 +107,32 @@ void require_ctx(csdr_context* ctx) {
 using namespace csdr;
 
 namespace {
+// Bytes of device memory that a product reads or writes.
+struct Extent {
+    uintptr_t lo, hi;
+    static Extent of(const void* p, size_t bytes) { return {reinterpret_cast<uintptr_t>(p), reinterpret_cast<uintptr_t>(p) + bytes}; }
+    bool meets(const Extent& o) const { return lo < o.hi && o.lo < hi; }
+    bool meets(const std::vector<Extent>& others) const {
+        return std::any_of(others.begin(), others.end(), [&](const Extent& o) { return meets(o); });
+    }
+};
+
 // A list the list kernel does not take: runs of independent products of one width and form on the
 // fp32 projection share their launches (seven 6711 x 545 at one token: 50 us one by one, 13 here), the rest go
-// one at a time.
+// one at a time. A run projects all its members before it gathers any, so a product joins only where
+// the outcome is that of the list taken in order: it reads nothing the run writes, and writes nothing
+// the run writes or reads. Runs end at what one projection launch holds.
 void launch_products(csdr_context* ctx, const std::vector<QueueItem>& items) {
     std::vector<const csdr_segment*> segs;
     std::vector<MatmulArgs> args;
+    std::vector<Extent> reads, writes;
     auto flush = [&] {
         if (segs.size() == 1) launch_matmul(ctx, segs[0], args[0]);
         else if (!segs.empty()) matmul_rows_simt(ctx, segs.data(), args.data(), static_cast<uint32_t>(segs.size()));
         segs.clear();
         args.clear();
+        reads.clear();
+        writes.clear();
     };
     for (const QueueItem& it : items) {
         MatmulArgs a;
@@ -128,12 +144,19 @@ void launch_products(csdr_context* ctx, const std::vector<QueueItem>& items) {
         a.y_layout = it.y_layout;
         a.bias = it.bias;
         const bool simt = it.batch > 0 && !tcgen05_supported(ctx, it.seg, it.batch) && simt_rows_supported(ctx, it.seg, it.batch);
-        const bool joins = simt && it.dep < 0 && !segs.empty() && segs[0]->g.cols == it.seg->g.cols && args[0].batch == a.batch &&
-                           args[0].x_dtype == a.x_dtype && args[0].x_layout == a.x_layout && args[0].y_layout == a.y_layout;
+        const Extent x = Extent::of(a.x, it.batch * it.seg->g.cols * (a.x_dtype == CSDR_DTYPE_BF16 ? 2u : 4u));
+        const Extent bias = Extent::of(a.bias, a.bias ? it.seg->g.rows * static_cast<size_t>(4) : 0u);
+        const Extent y = Extent::of(a.y, it.batch * it.seg->g.rows * static_cast<size_t>(4));
+        const bool joins = simt && it.dep < 0 && !segs.empty() && segs.size() < kSimtMembers && segs[0]->g.cols == it.seg->g.cols &&
+                           args[0].batch == a.batch && args[0].x_dtype == a.x_dtype && args[0].x_layout == a.x_layout &&
+                           args[0].y_layout == a.y_layout && !x.meets(writes) && !bias.meets(writes) && !y.meets(writes) && !y.meets(reads);
         if (!joins) flush();
         if (simt) {
             segs.push_back(it.seg);
             args.push_back(a);
+            reads.push_back(x);
+            reads.push_back(bias);
+            writes.push_back(y);
         } else {
             launch_matmul(ctx, it.seg, a);
         }
@@ -701,7 +724,13 @@ int csdr_matmul_group_device_async(csdr_context* ctx, const csdr_segment* const*
         size_t dictionary = 0;
         for (size_t i = 0; i < n_segs; ++i) dictionary += static_cast<size_t>(segs[i]->g.n_atoms) * segs[i]->g.cols;
         bool simt = batch > 0;
-        for (size_t i = 0; i < n_segs; ++i) simt = simt && simt_rows_supported(ctx, segs[i], batch, dictionary);
+        std::vector<Extent> held{Extent::of(x_dev, batch * segs[0]->g.cols * (x_dtype == CSDR_DTYPE_BF16 ? 2u : 4u))};
+        for (size_t i = 0; i < n_segs && simt; ++i) {
+            // members that overwrite the activations or each other's results keep the order they were given in
+            const Extent y = Extent::of(ys_dev[i], batch * segs[i]->g.rows * static_cast<size_t>(4));
+            simt = simt_rows_supported(ctx, segs[i], batch, dictionary) && !y.meets(held);
+            held.push_back(y);
+        }
         if (simt) {
             // fp32 projections of every member in one launch: two 5533 x 8468 at 6 tokens 62 us on the
             // one-launch GEMV, 22 here; three 3362 x 2292 of 128 atoms at 16 tokens 33 and 11
