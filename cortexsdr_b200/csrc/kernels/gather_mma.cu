@@ -19,9 +19,9 @@
 // warps about 600 cycles from the release of its buffer, the products of a block 384), warps 10-17 take
 // finished 128 x 192 accumulators (two, in tensor memory) out: a lane is a row, so token-major results
 // leave in 128-byte pieces.
-// A token whose projection is not finite comes out as NaN in every row (a zero coefficient times
-// infinity); its activations were not finite, and the two-piece products of the projection leave no
-// atom of such a token finite.
+// A projection that is not finite (an atom that is not, or a sum past fp32) belongs only into the rows
+// that name its atom, but a zero coefficient times it is NaN in every row: results that come out not
+// finite are worked out once more from the row's codes, as the lookups have them.
 // Every wait is bounded; one that runs out sets the status word and every role leaves.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -168,13 +168,33 @@ coefficient_entries_kernel(const uint16_t* __restrict__ codes, const float* __re
 struct GatherMmaParams {
     const uint32_t* entries;
     const uint32_t* starts;
-    uint32_t R, n_tiles, n_blocks, M, per_slice;
+    const uint16_t* codes;
+    const float* scales;
+    const __nv_bfloat16* planes;      // hi | mid | lo, each [K][stride]
+    uint32_t stride;
+    uint32_t R, S, k, n_tiles, n_blocks, M, per_slice;
     YView y;
     const float* residual;
     TokenScale ts;
     int* status;
     uint32_t spin;
 };
+
+// One result from the row's codes. Rare: a sum that is not finite.
+__device__ __noinline__ float looked_up(const GatherMmaParams& p, uint32_t row, uint32_t tok) {
+    const size_t plane = static_cast<size_t>(p.n_blocks) * kAtomBlock * p.stride;
+    const uint16_t* c = p.codes + static_cast<size_t>(row) * p.S * p.k;
+    float sum = 0.0f;
+    for (uint32_t s = 0; s < p.S * p.k; ++s) {
+        const uint32_t code = c[s];
+        const float gamma = p.scales[s / p.k];
+        const __nv_bfloat16* at = p.planes + static_cast<size_t>(code & 0x7FFFu) * p.stride + tok;
+        float v = __bfloat162float(at[0]);
+        if (isfinite(v)) v += __bfloat162float(at[plane]) + __bfloat162float(at[2u * plane]);
+        sum += __fmul_rn((code & 0x8000u) ? -gamma : gamma, v);
+    }
+    return sum;
+}
 
 // grid (per_slice CTAs over the row tiles, 64-token slices)
 __global__ void __launch_bounds__(kGmThreads, 1)
@@ -386,9 +406,19 @@ hsdr_gather_mma_kernel(const __grid_constant__ CUtensorMap map, const __grid_con
                     for (uint32_t j = 0; j < 16u; ++j) h[j] = 0.0f;
                 }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                float sum[16], odd = 0.0f;
 #pragma unroll
-                for (uint32_t j = 0; j < 16u; ++j)
-                    h[j] += fmaf(__uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j])), inv_s[first + ch * 16u + j], bias);
+                for (uint32_t j = 0; j < 16u; ++j) {
+                    sum[j] = __uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j]));
+                    odd = fmaf(sum[j], 0.0f, odd);          // NaN where a sum is not finite
+                }
+                if (odd != 0.0f) {
+#pragma unroll
+                    for (uint32_t j = 0; j < 16u; ++j)
+                        if (j < n && !isfinite(sum[j])) sum[j] = looked_up(p, row, t0 + first + ch * 16u + j);
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < 16u; ++j) h[j] += fmaf(sum[j], inv_s[first + ch * 16u + j], bias);
                 if (quads) {
 #pragma unroll
                     for (uint32_t j = 0; j < 16u; j += 4u) *reinterpret_cast<float4*>(dst + j) = make_float4(h[j], h[j + 1], h[j + 2], h[j + 3]);
@@ -502,7 +532,13 @@ void launch_gather_mma(csdr_context* ctx, const csdr_segment* seg, const DxPlane
     const Geometry& g = seg->g;
     GatherMmaParams p{};
     p.entries = entries_of(ctx, seg, &p.starts);
+    p.codes = seg->codes_ptr();
+    p.scales = static_cast<const float*>(seg->scales->ptr);
+    p.planes = dx.p;
+    p.stride = dx.stride;
     p.R = g.rows;
+    p.S = g.n_stages;
+    p.k = g.k;
     p.n_tiles = (g.rows + kRowsTile - 1u) / kRowsTile;
     p.n_blocks = g.n_atoms / kAtomBlock;
     p.M = M;

@@ -185,6 +185,13 @@ __device__ __forceinline__ void stamp(const Params& p, int slot) {
     }
 }
 
+// Two values towards zero, the first in the low half.
+__device__ __forceinline__ __nv_bfloat162 bf16x2_cut(float a, float b) {
+    uint32_t d;
+    asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(b), "f"(a));
+    return *reinterpret_cast<const __nv_bfloat162*>(&d);
+}
+
 // How Dx leaves: floats [atom][token], floats [token][atom], or bf16 planes. Instances, because the
 // branches cost the short launches (8 and 64 tokens) 2 % where they were decided at run time.
 enum class DxForm { kFloats, kTokenMajor, kPlanes };
@@ -405,7 +412,9 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
         }
         const size_t o = static_cast<size_t>(atom) * p.dx_stride + tok;
         if constexpr (FORM == DxForm::kPlanes) {   // four tokens always: the rows are padded to whole eights
-            const __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x, v.y), h1 = __floats2bfloat162_rn(v.z, v.w);
+            // hi is cut off, not rounded: a value that bf16 cannot reach by rounding stays finite, and the
+            // remaining 16 bits are exact in mid and lo all the same
+            const __nv_bfloat162 h0 = bf16x2_cut(v.x, v.y), h1 = bf16x2_cut(v.z, v.w);
             const float r0 = v.x - __low2float(h0), r1 = v.y - __high2float(h0), r2 = v.z - __low2float(h1), r3 = v.w - __high2float(h1);
             const __nv_bfloat162 m0 = __floats2bfloat162_rn(r0, r1), m1 = __floats2bfloat162_rn(r2, r3);
             const __nv_bfloat162 l0 = __floats2bfloat162_rn(r0 - __low2float(m0), r1 - __high2float(m0));

@@ -77,3 +77,33 @@ def test_other_stage_scales(oracle, monkeypatch, decay):
     pay = synth.hsdr_payload(200, 128, n_atoms=128, k=8, decay=decay, seed=4)
     x = np.random.default_rng(1).normal(0, 1, (70, 128)).astype(np.float32)
     check(oracle, monkeypatch, [pay], x, "f32", True)
+
+
+@pytest.mark.parametrize("token", [False, True])
+def test_values_that_are_not_finite_stay_in_the_rows_that_name_them(monkeypatch, token):
+    """A bad atom, a projection past fp32, one past what bf16 rounds to, a bad token: the same infinities
+    and NaN as the lookups, and none elsewhere."""
+    rows, cols, atoms, m, big = 300, 192, 512, 150, 11
+    pay = bytearray(synth.hsdr_payload(rows, cols, n_atoms=atoms, k=8, seed=9))
+    d = np.frombuffer(pay, np.float32, atoms * cols, 36 + 4 * 3).reshape(atoms, cols)   # behind the header and the stage scales
+    d[7, 100] = np.inf
+    d[20:, :big] = 0
+    d[20, :big - 1] = 2.0 ** np.arange(127, 127 - big + 1, -1)      # their sum: 2^128 (1 - 2^-10)
+    d[21, 0] = 2.0 ** 127
+    x = np.random.default_rng(2).normal(0, 1, (m, cols)).astype(np.float32)
+    x[:, :big] = 0
+    x[70, :big] = 1                                    # finite in fp32, past bf16's rounding
+    x[71, 0] = 64                                      # past fp32
+    x[140, 50] = np.nan
+    got, _ = run(monkeypatch, "1", [bytes(pay)], x, "f32", token, None)
+    look, _ = run(monkeypatch, "0", [bytes(pay)], x, "f32", token, None)
+    codes = np.frombuffer(bytes(pay), np.uint16, rows * 24, 36 + 4 * 3 + 4 * atoms * cols).reshape(rows, 24) & 0x7FFF
+    clean = ~np.isin(codes, (7, 20, 21)).any(axis=1)
+    assert 100 < clean.sum() < rows
+    fine = np.ones(m, bool)
+    fine[140] = False
+    assert np.isfinite(look[0][np.ix_(fine, clean)]).all() and np.isnan(look[0][140]).all()
+    assert not np.isfinite(look[0][np.ix_(fine, (codes == 7).any(axis=1))]).any()
+    assert np.isfinite(look[0][70, (codes[:, 16:] == 20).any(axis=1) & ~(codes[:, :16] == 20).any(axis=1) & ~np.isin(codes, (7, 21)).any(axis=1)]).all()
+    # the same 24-bit projection, 24 exact terms in fp32
+    np.testing.assert_allclose(got[0], look[0], rtol=1e-4, atol=1e-6 * np.abs(x[fine]).max(), equal_nan=True)
