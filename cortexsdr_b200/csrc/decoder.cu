@@ -315,7 +315,7 @@ void attend(csdr_decoder* d, uint32_t li, uint32_t T, float* out, __nv_bfloat16*
     op_rope_cache(ctx, F(d->q), F(d->k), F(d->v), kc, vc, d->kv_dtype, I32(d->seq_of), I32(d->pos_of), T, d->QH_l, d->KVH_l,
                   c.head_dim, c.max_seq, c.rope_theta);
     // tokens that share a sequence are the tokens of one forward call: consecutive positions
-    if (!d->distinct_seqs && attention_prompt_supported(ctx, T, c.head_dim))
+    if (!d->distinct_seqs && attention_prompt_supported(ctx, T, d->QH_l, d->KVH_l, c.head_dim))
         op_attention_prompt(ctx, F(d->q), kc, vc, d->kv_dtype, I32(d->seq_of), I32(d->pos_of), T, d->QH_l, d->KVH_l, c.head_dim,
                             c.max_seq, out, hi, lo);
     else

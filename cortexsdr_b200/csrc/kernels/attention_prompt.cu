@@ -274,8 +274,9 @@ void launch_kv(csdr_context* ctx, const float* q, const void* kc, const void* vc
 // Short prompts stay with the kernel that has a CTA for every (token, head): at 128 tokens it takes
 // 25 us against 29 (32 heads of 128) and 15 against 19 (14 heads of 64), at 256 64 against 48 and 29
 // against 29, at 512 214 against 104 and 80 against 50.
-bool attention_prompt_supported(const csdr_context* ctx, uint32_t T, uint32_t HD) {
-    return (HD == 64u || HD == 128u) && T >= ctx->prompt_attention_min;
+// Row blocks are the grid's second dimension: 65535 of 64 (token, query head of a group) rows.
+bool attention_prompt_supported(const csdr_context* ctx, uint32_t T, uint32_t QH, uint32_t KVH, uint32_t HD) {
+    return (HD == 64u || HD == 128u) && T >= ctx->prompt_attention_min && static_cast<uint64_t>(T) * (QH / KVH) <= 65535ull * kQ;
 }
 
 void op_attention_prompt(csdr_context* ctx, const float* q, const void* kc, const void* vc, int kv_dtype, const int32_t* seq_of,

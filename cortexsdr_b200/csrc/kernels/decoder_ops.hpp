@@ -44,7 +44,7 @@ void op_attention_step(csdr_context* ctx, const float* q, const float* k_new, co
                        __nv_bfloat16* lo = nullptr);
 // Attention of a prompt: T tokens of ONE sequence at consecutive positions, rotated and in the cache
 // already (attention_prompt.cu). Same results as op_attention up to the order of fp32 sums.
-bool attention_prompt_supported(const csdr_context* ctx, uint32_t T, uint32_t HD);
+bool attention_prompt_supported(const csdr_context* ctx, uint32_t T, uint32_t QH, uint32_t KVH, uint32_t HD);
 void op_attention_prompt(csdr_context* ctx, const float* q, const void* kc, const void* vc, int kv_dtype, const int32_t* seq_of,
                          const int32_t* pos_of, uint32_t T, uint32_t QH, uint32_t KVH, uint32_t HD, uint32_t max_seq, float* out,
                          __nv_bfloat16* hi = nullptr, __nv_bfloat16* lo = nullptr);

@@ -512,7 +512,7 @@ bool gather_mma_supported(const csdr_context* ctx, const csdr_segment* seg, size
     const Geometry& g = seg->g;
     if (!ctx->gather_mma || !ctx->tensor_cores || !ctx->tma || !encode_fn()) return false;
     if (!g.row_tiles() || g.n_atoms % (2u * kAtomBlock) || g.n_atoms > kMaxBlocks * kAtomBlock || g.slots() > kMaxSlots) return false;
-    if (batch <= 16u || batch > 0xFFFFFFu) return false;
+    if (batch <= 16u || batch > 65535u * static_cast<size_t>(kTok)) return false;   // slices: the grid's second dimension
     // A CTA first takes in 384 bytes of planes per atom, and its fixed part has to be shared by enough
     // (row tile, slice) pairs. Whole products, lookups against this: 512 atoms of 4096, 11008 rows, 128
     // tokens 20.2 / 20.7 us, 256 30.1 / 26.7, 512 45.7 / 37.1; 1024 rows, 256 tokens (32 pairs) 19.3 /

@@ -250,18 +250,11 @@ simt_reduce_kernel(const float* __restrict__ part, uint32_t rows, uint32_t M, ui
     y.y[y_index(y, r, t)] = v + (y.bias ? y.bias[r] : 0.0f);
 }
 
-}  // namespace
+// At most kMostTokens tokens: their tiles are the grid's second dimension.
+constexpr uint32_t kMostTokens = 65535u * 64u;
 
-void launch_gemm_simt(csdr_context* ctx, const float* W, uint32_t rows, uint32_t cols, const XView& x, const YView& y,
-                      bool w_fresh) {
-    const SimtMember one{W, x.x, rows, 0u};
-    launch_gemm_simt_many(ctx, &one, 1, rows, cols, x, y, w_fresh);
-}
-
-void launch_gemm_simt_many(csdr_context* ctx, const SimtMember* members, uint32_t n_members, uint32_t rows, uint32_t cols, const XView& x,
-                           const YView& y, bool w_fresh) {
-    if (rows == 0 || x.M == 0) return;
-    if (n_members == 0 || n_members > kSimtMembers) throw Error(CSDR_ERR_LIMIT, "fp32 product: 1 to 16 members");
+void launch_tokens(csdr_context* ctx, const SimtMember* members, uint32_t n_members, uint32_t rows, uint32_t cols, const XView& x,
+                   const YView& y, bool w_fresh) {
     const bool swap = y.layout == CSDR_LAYOUT_TOKEN_MAJOR;
     const uint32_t tok = x.M <= 16u ? 16u : x.M <= 32u ? 32u : 64u;
     SimtParams p{};
@@ -320,6 +313,28 @@ void launch_gemm_simt_many(csdr_context* ctx, const SimtMember* members, uint32_
         LaunchScope ls(ctx, KC_DX);
         CSDR_CUDA(cudaLaunchKernelEx(&cfg, simt_reduce_kernel, static_cast<const float*>(p.part), rows, x.M, p.n_split, y));
         ls.done("simt_reduce_kernel");
+    }
+}
+
+}  // namespace
+
+void launch_gemm_simt(csdr_context* ctx, const float* W, uint32_t rows, uint32_t cols, const XView& x, const YView& y,
+                      bool w_fresh) {
+    const SimtMember one{W, x.x, rows, 0u};
+    launch_gemm_simt_many(ctx, &one, 1, rows, cols, x, y, w_fresh);
+}
+
+void launch_gemm_simt_many(csdr_context* ctx, const SimtMember* members, uint32_t n_members, uint32_t rows, uint32_t cols, const XView& x,
+                           const YView& y, bool w_fresh) {
+    if (rows == 0) return;
+    if (n_members == 0 || n_members > kSimtMembers) throw Error(CSDR_ERR_LIMIT, "fp32 product: 1 to 16 members");
+    for (uint64_t t = 0; t < x.M; t += kMostTokens) {
+        XView xt = x;
+        YView yt = y;
+        xt.b0 += static_cast<uint32_t>(t);
+        yt.b0 += static_cast<uint32_t>(t);
+        xt.M = yt.M = static_cast<uint32_t>(std::min<uint64_t>(kMostTokens, x.M - t));
+        launch_tokens(ctx, members, n_members, rows, cols, xt, yt, w_fresh);
     }
 }
 

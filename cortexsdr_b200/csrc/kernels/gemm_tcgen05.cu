@@ -1224,7 +1224,8 @@ bool simt_rows_supported(const csdr_context* ctx, const csdr_segment* seg, size_
     if (!g.row_tiles() || batch > 0xFFFFFFFFull || g.slots() > kWideMaxSlots || g.n_stages > 64u) return false;
     if (!dictionary) dictionary = static_cast<size_t>(g.n_atoms) * g.cols;
     if (g.cols % 4u == 0 && (batch < ctx->simt_min_batch || (batch <= 16u && dictionary < ctx->simt_min_dict))) return false;
-    if (batch > 16u) return gather_wide_smem(g.n_atoms) <= ctx->smem_optin;
+    // the wide gather's token slices are its grid's second dimension
+    if (batch > 16u) return gather_wide_smem(g.n_atoms) <= ctx->smem_optin && batch <= 65535u * static_cast<size_t>(kWideTokens);
     return group_gather_smem(ctx, g.rows, g.slots(), g.n_atoms) <= ctx->smem_optin;
 }
 
