@@ -181,10 +181,12 @@ void* csdr_context::scratch_get(int slot, size_t bytes) {
     return scratch[slot]->ptr;
 }
 
-void csdr_context::scratch_trim(int slot, size_t most) {
-    if (!scratch[slot] || scratch[slot]->bytes <= most) return;
-    CSDR_CUDA(cudaStreamSynchronize(stream));
-    scratch[slot].reset();
+void csdr_context::encoder_scratch_trim() noexcept {
+    for (int slot = kEncoderScratch; slot < kScratchSlots; ++slot)
+        if (scratch[slot] && scratch[slot]->bytes > (256u << 20)) {
+            (void)cudaStreamSynchronize(stream);   // work of a call that ended early may still use it
+            scratch[slot].reset();
+        }
 }
 
 bool csdr_context::capturing() const {

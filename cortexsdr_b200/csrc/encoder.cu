@@ -69,6 +69,13 @@ DevPtr scratch(csdr_context* ctx, int slot, size_t bytes) {
     return ctx->scratch[slot];
 }
 
+// Stands in every entry point: what an uncommonly large tensor needed is not kept for the next call,
+// however this one ends.
+struct Workspaces {
+    csdr_context* ctx;
+    ~Workspaces() { ctx->encoder_scratch_trim(); }
+};
+
 // fitHierarchicalKSVD (:494-607) on a pool of tiles resident on the device (one tensor's, or the
 // pooled tiles of several tensors as fitSharedDictionary :1446-1469 hands them in): dictionary
 // init, a coding pass, ksvd_iters rounds of (atom update, coding pass), the non-finite sweep.
@@ -158,6 +165,7 @@ int csdr_encode_codes(csdr_context* ctx, const float* tiles, size_t n_tiles, siz
         if (n_tiles > 0xFFFFFFFFull || tile_dim > 0xFFFFFFFFull) throw Error(CSDR_ERR_LIMIT, "too many tiles");
         const size_t n_codes = n_tiles * n_stages * k_per_stage;
         if (capacity < n_codes) throw Error(CSDR_ERR_BUFFER, "code buffer too small");
+        const Workspaces keep{ctx};
         DevPtr t = upload(ctx, tiles, n_tiles * tile_dim * 4);
         DevPtr d = upload(ctx, atoms, static_cast<size_t>(n_atoms) * tile_dim * 4);
         DevPtr g = upload(ctx, stage_scales, 4u * n_stages);
@@ -191,11 +199,12 @@ int csdr_hsdr_encode(csdr_context* ctx, const float* W, uint32_t rows, uint32_t 
         if (!payload_out || capacity < total) throw Error(CSDR_ERR_BUFFER, "payload buffer too small");
         uint8_t* out = static_cast<uint8_t*>(payload_out);
 
-        DevPtr tiles = scratch(ctx, 2, static_cast<size_t>(rows) * cols * 4);
+        const Workspaces keep{ctx};
+        DevPtr tiles = scratch(ctx, 11, static_cast<size_t>(rows) * cols * 4);
         ctx->copies().upload(tiles->ptr, W, static_cast<size_t>(rows) * cols * 4);
         if (!(tile_rows == 1 && tile_cols == cols)) {   // whole rows are tiles as they lie
             const DevPtr Wd = tiles;
-            tiles = scratch(ctx, 7, static_cast<size_t>(n_tiles) * T * 4);
+            tiles = scratch(ctx, 12, static_cast<size_t>(n_tiles) * T * 4);
             launch_extract_tiles(ctx, static_cast<const float*>(Wd->ptr), cols, tile_rows, tile_cols, n_rt, n_ct,
                                  static_cast<float*>(tiles->ptr));
         }
@@ -223,8 +232,6 @@ int csdr_hsdr_encode(csdr_context* ctx, const float* W, uint32_t rows, uint32_t 
         uint8_t* codes_at = dict_at + 4u * static_cast<size_t>(n_atoms) * T;
         ctx->copies().download(dict_at, D->ptr, 4u * static_cast<size_t>(n_atoms) * T);
         ctx->copies().download(codes_at, codes, n_codes * 2);
-        // what an uncommonly large tensor needed is not kept for the next call
-        for (int slot : {2, 7, 8, 9, 10}) ctx->scratch_trim(slot, 256u << 20);
         // raw strips: top-right, then bottom (:1185-1197)
         uint8_t* e = codes_at + 2u * n_codes;
         const size_t wr = static_cast<size_t>(cols - C_full) * 4;
@@ -267,6 +274,7 @@ int csdr_hsdr_encode_shared(csdr_context* ctx, const float* const* tensors, cons
         }
         if (!fits) throw Error(CSDR_ERR_BUFFER, "output buffers too small");
 
+        const Workspaces keep{ctx};
         // the tensors' tiles pooled in order (the uncapped pool of compressGroupedSegments, :2383-2390)
         DevPtr pool = std::make_shared<DeviceBuffer>(static_cast<size_t>(n_pool) * T * 4, ctx->device);
         std::vector<size_t> first(n_tensors);

@@ -100,15 +100,20 @@ struct csdr_context {
     int sm_count = 0;
     size_t smem_optin = 0;
     uint64_t launches = 0;
-    // Grow-only scratch (Dx partials, factored 2-D products, host staging).
     std::unique_ptr<csdr::HostCopier> copier;   // large copies of pageable memory; made on first use
     csdr::HostCopier& copies() {
         if (!copier) copier = std::make_unique<csdr::HostCopier>(device, stream);
         return *copier;
     }
-    csdr::DevPtr scratch[11];  // 0 Dx, 1 tile products, 2 materialised W, 3 host staging, 4 fused-GEMV partials, 5 activation planes / wait self-test, 6 GEMV queue, 7 dense product before re-tiling, 8 - 10 encoder (dictionary, codes and small arrays, projections)
+    // Scratch. 0 - 7 only grow, so that a captured graph keeps what it was captured with as long as no later
+    // call needs more: 0 Dx, 1 tile products, 2 materialised W, 3 host staging, 4 fused-GEMV partials,
+    // 5 activation planes / wait self-test, 6 GEMV queue, 7 dense product before re-tiling. The rest is the
+    // encoder's, which no graph holds: 8 dictionary, 9 codes and small arrays, 10 projections, 11 the
+    // matrix, 12 its tiles.
+    static constexpr int kEncoderScratch = 8, kScratchSlots = 13;
+    csdr::DevPtr scratch[kScratchSlots];
     void* scratch_get(int slot, size_t bytes);
-    void scratch_trim(int slot, size_t most);   // gives a slot back that has grown past `most` bytes
+    void encoder_scratch_trim() noexcept;       // at the end of an encoder call: keeps up to 256 MB a slot
     bool capturing() const;                     // the stream is being captured: nothing may be built on first use
     int* status_word = nullptr;  // device int: kernels record bounded-wait timeouts here
     // Page-locked, device-mapped host staging for the host-buffer entry points (grow-only).
