@@ -189,6 +189,21 @@ void csdr_context::encoder_scratch_trim() noexcept {
         }
 }
 
+csdr::DevPtr csdr_context::try_keep(size_t bytes) {
+    const size_t before = kept->fetch_add(bytes);
+    try {
+        if (bytes <= keep_budget && before <= keep_budget - bytes)
+            return DevPtr(new DeviceBuffer(bytes, device), [count = kept, bytes](DeviceBuffer* b) {
+                delete b;
+                count->fetch_sub(bytes);
+            });
+    } catch (const Error&) {
+        (void)cudaGetLastError();   // no room: the caller takes the form that needs none
+    }
+    kept->fetch_sub(bytes);
+    return nullptr;
+}
+
 bool csdr_context::capturing() const {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     CSDR_CUDA(cudaStreamIsCapturing(stream, &status));
@@ -282,6 +297,8 @@ int csdr_context_create(int device, void* stream, csdr_context** out) {
         ctx->device = device;
         ctx->sm_count = prop.multiProcessorCount;
         ctx->smem_optin = prop.sharedMemPerBlockOptin;
+        ctx->keep_budget = prop.totalGlobalMem / 4u;
+        if (const char* e = std::getenv("CSDR_KEEP_MB")) ctx->keep_budget = static_cast<size_t>(std::max(0, std::atoi(e))) << 20;
         if (stream) {
             ctx->stream = static_cast<cudaStream_t>(stream);
         } else {

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <memory>
 #include <mutex>
@@ -114,6 +115,11 @@ struct csdr_context {
     csdr::DevPtr scratch[kScratchSlots];
     void* scratch_get(int slot, size_t bytes);
     void encoder_scratch_trim() noexcept;       // at the end of an encoder call: keeps up to 256 MB a slot
+    // What a segment keeps although there is a form that does without it (a rebuilt weight, coefficient
+    // entries). Null where all of them together would pass the budget or the device has no room.
+    csdr::DevPtr try_keep(size_t bytes);
+    size_t keep_budget = 0;                     // bytes; CSDR_KEEP_MB, else a quarter of the device's memory
+    std::shared_ptr<std::atomic<size_t>> kept = std::make_shared<std::atomic<size_t>>(0);
     bool capturing() const;                     // the stream is being captured: nothing may be built on first use
     int* status_word = nullptr;  // device int: kernels record bounded-wait timeouts here
     // Page-locked, device-mapped host staging for the host-buffer entry points (grow-only).
@@ -132,7 +138,7 @@ struct csdr_context {
     csdr::DevPtr gemv_trace;  // when set: 8 global-timer stamps per CTA of the last fused GEMV
     bool fused_gemv = true;  // CSDR_FUSED_GEMV=0 selects the two-kernel path
     bool gemv_queue = true;  // CSDR_GEMV_QUEUE=0 keeps lists of products on single and grouped launches
-    bool cache_2d = true;            // CSDR_CACHE_2D=0: wide batches on 2-D tiles stay on the factored CUDA-core kernels
+    bool cache_2d = true;            // CSDR_CACHE_2D=0: 2-D tiles keep no rebuilt weight, at any batch
     uint32_t queue_poll_sleep_ns = 400;  // CSDR_QUEUE_POLL_SLEEP: pause between polls of the list kernel's dependent hand-overs
     uint32_t queue_min_group = 4;    // CSDR_QUEUE_MIN_GROUP: smallest same-x group the list kernel takes over grouped fused launches
     bool host_zero_copy = true;      // CSDR_HOST_ZERO_COPY=0: results of a host list go back by a copy even when the caller's memory is device-addressable
@@ -184,12 +190,12 @@ struct csdr_segment {
     // output row) whose cached bf16 planes feed the tensor-core kernel at wide batches - what the
     // reference's layer cache holds as fp32 after decompress(). Built on the first wide product.
     mutable std::shared_ptr<csdr_segment> dense;
-    // The same as fp32, for the shapes the tensor maps do not take.
+    // The same as fp32, for the shapes the tensor maps do not take (try_keep).
     mutable csdr::DevPtr dense_f32;
     // 2-D tile images only: the dictionary seen as n_atoms * tile_rows rows of tile_cols columns,
     // the shape in which the tensor-core projection computes all tile products of a few tokens.
     mutable std::shared_ptr<csdr_segment> tile_view;
-    // Row tiles: the codes as coefficient entries sorted by row tile and atom block (gather_mma.cu).
+    // Row tiles: the codes as coefficient entries sorted by row tile and atom block (gather_mma.cu; try_keep).
     mutable csdr::DevPtr coefficients;
     const uint16_t* codes_ptr() const {
         return static_cast<const uint16_t*>(codes->ptr) + codes_offset;

@@ -775,16 +775,19 @@ void launch_matmul(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs&
                                              a.batch * tile_words >= 8u * static_cast<size_t>(g.rows) ||
                                              a.batch * (tile_words + static_cast<size_t>(g.rows) * g.slots()) >=
                                                  static_cast<size_t>(g.rows) * g.tile_cols);
-    // (the rebuilt weight is made on first use: not while the stream is captured)
-    if (!g.row_tiles() && ctx->cache_2d && !planes_2d && dense_2d && (seg->dense_f32 || !ctx->capturing())) {
-        if (!seg->dense_f32) {
-            auto w = std::make_shared<DeviceBuffer>(static_cast<size_t>(g.rows) * g.cols * 4u, ctx->device);
-            launch_decode_rows(ctx, seg, nullptr, g.rows, static_cast<float*>(w->ptr));
-            CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
-            seg->dense_f32 = w;
+    if (!g.row_tiles() && ctx->cache_2d && !planes_2d && dense_2d) {
+        // the rebuilt weight is made on first use: not while the stream is captured, and only where there is room
+        if (!seg->dense_f32 && !ctx->capturing()) {
+            if (const DevPtr w = ctx->try_keep(static_cast<size_t>(g.rows) * g.cols * 4u)) {
+                launch_decode_rows(ctx, seg, nullptr, g.rows, static_cast<float*>(w->ptr));
+                CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
+                seg->dense_f32 = w;
+            }
         }
-        launch_dense_matmul(ctx, static_cast<const float*>(seg->dense_f32->ptr), g.rows, g.cols, a, false);
-        return;
+        if (seg->dense_f32) {
+            launch_dense_matmul(ctx, static_cast<const float*>(seg->dense_f32->ptr), g.rows, g.cols, a, false);
+            return;
+        }
     }
     const size_t budget = std::min<size_t>(ctx->smem_optin, 200u * 1024u);
     const bool fast_tiles = !fast_rows && (g.tile_cols % 4u == 0);
