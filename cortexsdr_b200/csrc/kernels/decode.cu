@@ -365,7 +365,9 @@ void launch_decode_rows(csdr_context* ctx, const csdr_segment* seg, const int32_
     // and whose atoms' slices fit shared memory: 64 elements of each up to 880 atoms, 32 up to 1760.
     const uint64_t T = g.tile_dim();
     const size_t smem64 = static_cast<size_t>(g.n_atoms) * 256u;
-    if (!rows_dev && n_rows == g.rows && g.n_tiles && T >= 32u && T <= 0x7FFFFFFFull && smem64 / 2u <= ctx->smem_optin &&
+    // (a tile's span in the matrix is counted in 32 bits)
+    const uint64_t span = g.tile_rows ? (g.tile_rows - 1ull) * g.cols + g.tile_cols : 0u;
+    if (!rows_dev && n_rows == g.rows && g.n_tiles && T >= 32u && T <= 0x7FFFFFFFull && span <= 0xFFFFFFFFull && smem64 / 2u <= ctx->smem_optin &&
         static_cast<uint64_t>(g.n_tiles) * g.slots() >= 2ull * g.n_atoms) {
         const bool wide = smem64 <= ctx->smem_optin;
         const size_t smem = wide ? smem64 : smem64 / 2u;
