@@ -262,7 +262,7 @@ hsdr_gather_mma_kernel(const __grid_constant__ CUtensorMap map, const __grid_con
         uint32_t phase = 0;                                // of both buffers: nb is even
         for (uint32_t ti = 0; ti < hi - lo && ok; ++ti) {
             const uint32_t acc = ti & 1u, d = tmem_base + acc * 256u;
-            if (ti >= 2u) ok = mbar_wait(smem_u32(&acc_empty[acc]), (ti / 2u - 1u) & 1u, p.spin, failed);
+            if (ti >= 2u) ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&acc_empty[acc]), (ti / 2u - 1u) & 1u, p.spin, failed));
             uint32_t b_lo = b_lo0;
             for (uint32_t b = 0; b < nb && ok; b += 2u, phase ^= 1u) {
 #pragma unroll

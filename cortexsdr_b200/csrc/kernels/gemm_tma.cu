@@ -686,7 +686,7 @@ hsdr_tile_project_mma_kernel(const __grid_constant__ CUtensorMap map_hi, const _
         uint32_t s = 0, parity = 0, at = ring_lo;
         for (uint32_t ti = 0; ti < mine && ok; ++ti) {
             const uint32_t acc = ti & 1u, d = tmem_base + acc * N;
-            if (ti >= 2u) ok = mbar_wait(smem_u32(&acc_empty[acc]), (ti / 2u - 1u) & 1u, p.spin);
+            if (ti >= 2u) ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&acc_empty[acc]), (ti / 2u - 1u) & 1u, p.spin));
             for (uint32_t kb = 0; kb < p.n_kb && ok; ++kb) {
                 ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&full_bar[s]), parity, p.spin) && !failed_s);
                 if (!ok) break;

@@ -47,3 +47,16 @@ def test_device_waits_are_bounded():
                 unbounded.append(f"{f}:{n + 1}")
     assert sites >= 4          # the check sees the waits it is meant to see
     assert unbounded == []
+
+
+def test_warps_leave_waits_together():
+    # a wait that a whole warp branches on is voted on, there or on the next line: lanes that gave up one
+    # by one would part ways with those that meet them at the next vote
+    kdir = os.path.join(ROOT, "cortexsdr_b200", "csrc", "kernels")
+    alone = []
+    for f in ("gather_mma.cu", "gemm_tma.cu"):
+        lines = open(os.path.join(kdir, f), errors="replace").read().splitlines()
+        for n, line in enumerate(lines):
+            if re.search(r"\b(ok|live)\b = .*mbar_wait\(", line) and "__all_sync" not in line + lines[n + 1]:
+                alone.append(f"{f}:{n + 1}: {line.strip()}")
+    assert alone == []
