@@ -365,8 +365,12 @@ hsdr_tile_gather_kernel(const uint16_t* __restrict__ codes, uint32_t Tr, uint32_
     const uint32_t jl = tid & 31u, grp = tid >> 5;
     const uint32_t j = jc * 32u + jl;
     float acc[MT];
+    size_t tok[MT];       // products of tokens the chunk does not have need not exist: the last one's again
 #pragma unroll
-    for (int b = 0; b < MT; ++b) acc[b] = 0.0f;
+    for (int b = 0; b < MT; ++b) {
+        acc[b] = 0.0f;
+        tok[b] = min(static_cast<uint32_t>(b), yv.M - 1u) * ps.token;
+    }
     if (j < Tr) {
         for (uint32_t bc = crank * 8u + grp; bc < n_ct; bc += 8u * csize) {
             const uint16_t* tc = cs + bc * slots;
@@ -383,7 +387,7 @@ hsdr_tile_gather_kernel(const uint16_t* __restrict__ codes, uint32_t Tr, uint32_
                     scale[q] = s0 + q < slots ? ((code & 0x8000u) ? -gamma : gamma) : 0.0f;
                     const float* p = pb + static_cast<size_t>(code & 0x7FFFu) * ps.atom;
 #pragma unroll
-                    for (int b = 0; b < MT; ++b) v[q][b] = __ldg(p + static_cast<size_t>(b) * ps.token);
+                    for (int b = 0; b < MT; ++b) v[q][b] = __ldg(p + tok[b]);
                 }
 #pragma unroll
                 for (int q = 0; q < 8; ++q)

@@ -56,3 +56,17 @@ def test_wide_products_token_major(ctx, oracle, rows, cols, m, shift):
     got, xd = product(ctx, pay, x, "f32", True, shift)
     want = xd @ oracle.decompress(pay).astype(np.float64).T
     assert np.linalg.norm(got - want) <= SPLIT * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("m", [3, 7, 11, 15])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_chunks_of_three_tokens(oracle, dtype, m):
+    """The gather's last chunk holds three tokens in a place for four; the products of the fourth would
+    lie behind the tile products (10 MB a chunk, in a context that has no larger scratch)."""
+    ctx = cs.Context(0)
+    pay = synth.hsdr_payload(640, 1664, tile_rows=128, tile_cols=128, n_atoms=512, k=5, seed=m)
+    x = np.random.default_rng(m).normal(0, 1, (m, 1664)).astype(np.float32)
+    got, xd = product(ctx, pay, x, dtype, True)
+    want = xd @ oracle.decompress(pay).astype(np.float64).T
+    assert np.linalg.norm(got - want) <= SPLIT * np.linalg.norm(want)
+    ctx.close()
