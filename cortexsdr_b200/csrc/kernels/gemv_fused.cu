@@ -120,22 +120,23 @@ __device__ __forceinline__ void stage_x(const XView& xv, uint32_t c0, uint32_t c
 //   xs      [MT][xcols]    activations (xcols = C when they fit, else one column slab)
 //   codes   per segment: the CTA's rows of the code stream, 16-byte units
 //   scales  per segment: S floats (padded to 4)
-//   dxs     [K][MTG]       Dx slices: of every segment side by side where they fit, else of one at a time
+//   dxs     [K][MTG]       Dx slices: of one segment at a time, or of every segment side by side (TOGETHER)
 struct SmemPlan {
     uint32_t xcols;                       // C (whole x resident) or slab
     uint32_t codes_off[kMaxFusedGroup];   // byte offsets
     uint32_t scales_off[kMaxFusedGroup];
     uint32_t dxs_off;
-    uint32_t dxs_segs;                    // segments whose slices lie side by side
     uint32_t k_off[kMaxFusedGroup + 1];   // atoms of the segments before
     uint32_t normw_off;                   // the norm weights of the folded normalisation, [C]
 };
 
 // Register budget: two launches must be able to sit on an SM together (two CTAs each), or the
 // next launch's weight prefetch cannot start before this one retires.
-// MULTI: more than one segment (what places an element or a row among several costs a single product
-// 0.4 us of its 5.9).
-template <int MT, int A, int U, bool MULTI>
+// TOGETHER: the segments of a group are handed over and their rows walked together, with one barrier
+// between (a CTA has 16 rows of a 4864-row segment for its 256 threads: gate and up of 4864 x 896 7.5 us
+// against 8.4 one after the other). What places an element or a row among several costs a single product
+// 0.4 us of its 5.9 and is in this instance only.
+template <int MT, int A, int U, bool TOGETHER>
 __global__ void __launch_bounds__(kThreads, (MT <= 4 ? 4 : 3))
 hsdr_gemv_fused_kernel(const __grid_constant__ FusedParams p, const __grid_constant__ SmemPlan plan) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -207,7 +208,7 @@ hsdr_gemv_fused_kernel(const __grid_constant__ FusedParams p, const __grid_const
             const FusedSeg& sg = p.seg[si];
             const uint32_t row0 = rchunk * sg.rows_per_cta;
             rows_before += row0 < sg.R ? min(sg.rows_per_cta, sg.R - row0) : 0u;
-            if (MULTI && tid == 0) r_off_s[si + 1u] = rows_before;
+            if (TOGETHER && tid == 0) r_off_s[si + 1u] = rows_before;
             if (row0 < sg.R) {
                 const uint32_t rows_here = min(sg.rows_per_cta, sg.R - row0);
                 const uint32_t slots = sg.S * sg.k;
@@ -346,130 +347,141 @@ hsdr_gemv_fused_kernel(const __grid_constant__ FusedParams p, const __grid_const
     // a wait that ran out earlier on this context (or in this launch) is not repeated
     uint32_t limit = *reinterpret_cast<const volatile int*>(p.status) != 0 ? 0u : p.spin_limit;
     const unsigned long long want_tag = static_cast<unsigned long long>(epoch) << 32;
-    // All segments at once where their Dx slices fit shared memory side by side (plan.dxs_segs), else one
-    // after the other: one hand-over, one barrier, and the rows of all of them walked together (a CTA has
-    // 16 rows of a 4864-row segment for its 256 threads).
-    for (uint32_t s0 = 0; s0 < (MULTI ? p.n_seg : 1u); s0 += MULTI ? plan.dxs_segs : 1u) {
-        const uint32_t s1 = MULTI ? min(p.n_seg, s0 + plan.dxs_segs) : 1u;
-        const uint32_t n_k = MULTI ? plan.k_off[s1] - plan.k_off[s0] : p.seg[0].K;
-        const uint32_t one_row0 = rchunk * p.seg[0].rows_per_cta;
-        const uint32_t n_rows = MULTI ? r_off_s[s1] - r_off_s[s0]
-                                      : one_row0 < p.seg[0].R ? min(p.seg[0].rows_per_cta, p.seg[0].R - one_row0) : 0u;
-        if (n_rows) {
-            // -- hand-over: poll this token group's partial words, 16 loads in flight --
-            const uint32_t n_el = n_k * MTG;                        // dxs elements
-            const uint32_t mine_el = tid < n_el ? (n_el - tid + kThreads - 1u) / kThreads : 0u;
-            const uint32_t n_w = mine_el * p.nsplit;               // words this thread owns
-            uint32_t j0 = 0, sp0 = 0;                              // (element ordinal, split) of word w0
-            for (uint32_t w0 = 0; w0 < n_w; w0 += 16u) {
-                unsigned long long e[16];
-                for (uint32_t spins = 0;; ++spins) {
-                    uint32_t j = j0, sp = sp0;
-                    bool ok = true;
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) {
-                        if (w0 + q < n_w) {
-                            const uint32_t el = tid + j * kThreads;
-                            const uint32_t ag = el / MTG, b = el - ag * MTG;
-                            uint32_t si = s0;
-                            if constexpr (MULTI)
-                                while (si + 1u < s1 && ag >= plan.k_off[si + 1u] - plan.k_off[s0]) ++si;
-                            const FusedSeg& sg = p.seg[MULTI ? si : 0u];
-                            const uint32_t a = MULTI ? ag - (plan.k_off[si] - plan.k_off[s0]) : ag;
-                            e[q] = ld_poll(p.part + sg.part_off + (static_cast<size_t>(sp) * sg.K + a) * MT + tg * MTG + b);
-                            if (++sp == p.nsplit) {
-                                sp = 0;
-                                ++j;
-                            }
-                        } else {
-                            e[q] = want_tag;
-                        }
-                    }
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) ok = ok && static_cast<uint32_t>(e[q] >> 32) == epoch;
-                    if (ok) break;
-                    if (spins >= limit) {  // gave up: the host will see it; nothing after this waits
-                        late = true;
-                        limit = 0u;
-                        break;
-                    }
-                }
+    // Hand-over: polls this token group's partial words, 16 loads in flight, and adds them up into n_k atoms'
+    // Dx slices; word(split, atom) is where a token group's words lie.
+    auto hand_over = [&](uint32_t n_k, auto word) {
+        const uint32_t n_el = n_k * MTG;                        // dxs elements
+        const uint32_t mine_el = tid < n_el ? (n_el - tid + kThreads - 1u) / kThreads : 0u;
+        const uint32_t n_w = mine_el * p.nsplit;               // words this thread owns
+        uint32_t j0 = 0, sp0 = 0;                              // (element ordinal, split) of word w0
+        for (uint32_t w0 = 0; w0 < n_w; w0 += 16u) {
+            unsigned long long e[16];
+            for (uint32_t spins = 0;; ++spins) {
+                uint32_t j = j0, sp = sp0;
+                bool ok = true;
 #pragma unroll
                 for (int q = 0; q < 16; ++q) {
                     if (w0 + q < n_w) {
-                        const uint32_t el = tid + j0 * kThreads;
-                        const float prev = sp0 ? dxs[el] : 0.0f;  // split order, whatever the batch boundaries
-                        dxs[el] = prev + __uint_as_float(static_cast<uint32_t>(e[q]));
-                        if (++sp0 == p.nsplit) {
-                            sp0 = 0;
-                            ++j0;
+                        const uint32_t el = tid + j * kThreads;
+                        const uint32_t a = el / MTG, b = el - a * MTG;
+                        e[q] = ld_poll(word(sp, a) + tg * MTG + b);
+                        if (++sp == p.nsplit) {
+                            sp = 0;
+                            ++j;
                         }
+                    } else {
+                        e[q] = want_tag;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 16; ++q) ok = ok && static_cast<uint32_t>(e[q] >> 32) == epoch;
+                if (ok) break;
+                if (spins >= limit) {  // gave up: the host will see it; nothing after this waits
+                    late = true;
+                    limit = 0u;
+                    break;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                if (w0 + q < n_w) {
+                    const uint32_t el = tid + j0 * kThreads;
+                    const float prev = sp0 ? dxs[el] : 0.0f;  // split order, whatever the batch boundaries
+                    dxs[el] = prev + __uint_as_float(static_cast<uint32_t>(e[q]));
+                    if (++sp0 == p.nsplit) {
+                        sp0 = 0;
+                        ++j0;
                     }
                 }
             }
         }
-        __syncthreads();  // dxs complete; first pass: also the cp.async fills
-        if (s0 == 0) stamp(p, 5);
-        const uint32_t b = tid % MTG, tok = tg * MTG + b;
-        auto walk = [&](uint32_t si, uint32_t rl) {
-            const FusedSeg& sg = p.seg[MULTI ? si : 0u];
-            const uint32_t row0 = rchunk * sg.rows_per_cta, slots = sg.S * sg.k;
-            const uint32_t skip = static_cast<uint32_t>((static_cast<size_t>(row0) * slots * 2u) & 15u) >> 1;
-            const uint16_t* rc = reinterpret_cast<const uint16_t*>(smem_raw + plan.codes_off[si]) + skip + rl * slots;
-            const float* sc = reinterpret_cast<const float*>(smem_raw + plan.scales_off[si]);
-            const float* dx = dxs + (MULTI ? (plan.k_off[si] - plan.k_off[s0]) * MTG : 0u) + b;
-            // what the epilogue adds comes from global memory and does not depend on the sum:
-            // requested here, it arrives while the codes are walked
-            const uint32_t r = row0 + rl;
-            const bool live = tok < sg.y.M;
-            const size_t yi = live ? y_index(sg.y, r, tok) : 0;
-            const float bias_v = live && sg.y.bias ? sg.y.bias[r] : 0.0f;
-            const float resid_v = live && sg.y.residual ? sg.y.residual[yi] : 0.0f;
-            float accr = 0.0f;
-            for (uint32_t l = 0; l < sg.S; ++l) {
-                const float gamma = sc[l];
-                const uint16_t* lc = rc + l * sg.k;
-                for (uint32_t k0 = 0; k0 < sg.k; k0 += 8u) {
-                    // eight independent lookups in flight, then the adds in slot order
-                    float t[8];
+    };
+    // One row of segment si: r its row, rc its codes, dx the segment's slice.
+    auto finish = [&](const FusedSeg& sg, uint32_t si, uint32_t r, const uint16_t* rc, const float* sc, const float* dx) {
+        const uint32_t b = tid % MTG;
+        // what the epilogue adds comes from global memory and does not depend on the sum:
+        // requested here, it arrives while the codes are walked
+        const uint32_t tok = tg * MTG + b;
+        const bool live = tok < sg.y.M;
+        const size_t yi = live ? y_index(sg.y, r, tok) : 0;
+        const float bias_v = live && sg.y.bias ? sg.y.bias[r] : 0.0f;
+        const float resid_v = live && sg.y.residual ? sg.y.residual[yi] : 0.0f;
+        float accr = 0.0f;
+        for (uint32_t l = 0; l < sg.S; ++l) {
+            const float gamma = sc[l];
+            const uint16_t* lc = rc + l * sg.k;
+            for (uint32_t k0 = 0; k0 < sg.k; k0 += 8u) {
+                // eight independent lookups in flight, then the adds in slot order
+                float t[8];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const uint32_t code = k0 + q < sg.k ? lc[k0 + q] : 0u;
-                        const float v = dx[(code & 0x7FFFu) * MTG];
-                        t[q] = __fmul_rn((code & 0x8000u) ? -gamma : gamma, v);
-                    }
+                for (int q = 0; q < 8; ++q) {
+                    const uint32_t code = k0 + q < sg.k ? lc[k0 + q] : 0u;
+                    const float v = dx[(code & 0x7FFFu) * MTG + b];
+                    t[q] = __fmul_rn((code & 0x8000u) ? -gamma : gamma, v);
+                }
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        if (k0 + q < sg.k) accr = __fadd_rn(accr, t[q]);
-                }
-            }
-            if (live) {
-                if (p.norm_w) accr *= inv_s[tok];
-                if (sg.y.bias) accr += bias_v;
-                if (MULTI && p.swiglu && si == 1u) {
-                    // silu_mul (api/cortex_sdk.cpp:1245-1256); this thread wrote the gate row itself
-                    const float gv = p.seg[0].y.y[yi];
-                    accr = (gv * (1.0f / (1.0f + expf(-gv)))) * accr;
-                }
-                if (sg.y.residual) accr += resid_v;
-                sg.y.y[yi] = accr;
-            }
-        };
-        constexpr uint32_t RP = kThreads / MTG;
-        if (!MULTI) {
-            for (uint32_t rl = tid / MTG; rl < n_rows; rl += RP) walk(0u, rl);
-        } else if (p.swiglu) {
-            // a thread takes a row of both: equal rows, one behind the other
-            for (uint32_t rl = tid / MTG; rl < (s1 - s0 == 2u ? n_rows / 2u : n_rows); rl += RP)
-                for (uint32_t si = s0; si < s1; ++si) walk(si, rl);
-        } else {
-            for (uint32_t v = tid / MTG; v < n_rows; v += RP) {
-                uint32_t si = s0;
-                while (si + 1u < s1 && v >= r_off_s[si + 1u] - r_off_s[s0]) ++si;
-                walk(si, v - (r_off_s[si] - r_off_s[s0]));
+                for (int q = 0; q < 8; ++q)
+                    if (k0 + q < sg.k) accr = __fadd_rn(accr, t[q]);
             }
         }
-        if (MULTI) __syncthreads();  // dxs is rewritten for the next segments
+        if (live) {
+            if (p.norm_w) accr *= inv_s[tok];
+            if (sg.y.bias) accr += bias_v;
+            if (p.swiglu && si == 1u) {
+                // silu_mul (api/cortex_sdk.cpp:1245-1256); this thread wrote the gate row itself
+                const float gv = p.seg[0].y.y[yi];
+                accr = (gv * (1.0f / (1.0f + expf(-gv)))) * accr;
+            }
+            if (sg.y.residual) accr += resid_v;
+            sg.y.y[yi] = accr;
+        }
+    };
+    auto codes_of = [&](const FusedSeg& sg, uint32_t si) {      // this CTA's rows of a segment
+        const uint32_t skip = static_cast<uint32_t>((static_cast<size_t>(rchunk * sg.rows_per_cta) * (sg.S * sg.k) * 2u) & 15u) >> 1;
+        return reinterpret_cast<const uint16_t*>(smem_raw + plan.codes_off[si]) + skip;
+    };
+    auto scales_of = [&](uint32_t si) { return reinterpret_cast<const float*>(smem_raw + plan.scales_off[si]); };
+    constexpr uint32_t RP = kThreads / MTG;
+    if constexpr (TOGETHER) {
+        const uint32_t n_rows = r_off_s[p.n_seg];
+        if (n_rows)
+            hand_over(plan.k_off[p.n_seg], [&](uint32_t sp, uint32_t a) {
+                uint32_t si = 0;
+                while (si + 1u < p.n_seg && a >= plan.k_off[si + 1u]) ++si;
+                const FusedSeg& sg = p.seg[si];
+                return p.part + sg.part_off + (static_cast<size_t>(sp) * sg.K + a - plan.k_off[si]) * MT;
+            });
+        __syncthreads();  // dxs and the cp.async fills complete
+        stamp(p, 5);
+        // SwiGLU: a thread takes a row of both, equal rows, one behind the other
+        const uint32_t pair = p.swiglu ? 2u : 1u;
+        for (uint32_t v = tid / MTG; v < n_rows / pair; v += RP) {
+            uint32_t si = 0;
+            while (pair == 1u && si + 1u < p.n_seg && v >= r_off_s[si + 1u]) ++si;
+            const uint32_t rl = v - r_off_s[si];
+            for (uint32_t i = 0; i < pair; ++i) {
+                const FusedSeg& sg = p.seg[si + i];
+                finish(sg, si + i, rchunk * sg.rows_per_cta + rl, codes_of(sg, si + i) + rl * (sg.S * sg.k), scales_of(si + i),
+                       dxs + plan.k_off[si + i] * MTG);
+            }
+        }
+    } else {
+        for (uint32_t si = 0; si < p.n_seg; ++si) {
+            const FusedSeg& sg = p.seg[si];
+            const uint32_t row0 = rchunk * sg.rows_per_cta;
+            if (row0 < sg.R) {
+                const unsigned long long* part = p.part + sg.part_off;
+                hand_over(sg.K, [&](uint32_t sp, uint32_t a) { return part + (static_cast<size_t>(sp) * sg.K + a) * MT; });
+            }
+            __syncthreads();  // dxs complete; first pass: also the cp.async fills
+            if (si == 0) stamp(p, 5);
+            if (row0 < sg.R) {
+                const uint32_t rows_here = min(sg.rows_per_cta, sg.R - row0), slots = sg.S * sg.k;
+                const uint16_t* cs = codes_of(sg, si);
+                for (uint32_t rl = tid / MTG; rl < rows_here; rl += RP) finish(sg, si, row0 + rl, cs + rl * slots, scales_of(si), dxs);
+            }
+            if (si + 1u < p.n_seg) __syncthreads();  // dxs is rewritten for the next segment
+        }
     }
     if (late) atomicExch(p.status, 1);
     // CTA 0 (always a gather CTA) retires the launch's tag: every CTA has read it long ago
@@ -480,7 +492,6 @@ hsdr_gemv_fused_kernel(const __grid_constant__ FusedParams p, const __grid_const
 
 template <int MT, int A, int U>
 void launch_t(csdr_context* ctx, FusedParams& p, uint32_t max_k, bool pdl) {
-    auto kern = p.n_seg > 1u ? hsdr_gemv_fused_kernel<MT, A, U, true> : hsdr_gemv_fused_kernel<MT, A, U, false>;
     // Activations stay whole in shared memory when they are small; otherwise one slab at a time.
     SmemPlan plan{};
     constexpr uint32_t token_groups = MT <= 4 ? 1u : MT / 4u;
@@ -489,13 +500,20 @@ void launch_t(csdr_context* ctx, FusedParams& p, uint32_t max_k, bool pdl) {
     // smallest grid this kernel can get (one CTA per SM), then launch with what fits.
     uint32_t all_k = 0;
     for (uint32_t i = 0; i < p.n_seg; ++i) all_k += p.seg[i].K;
-    // Side by side as long as the slices leave room for two CTAs on an SM, and only where every CTA has at
-    // most one projection task: where they have more, the rows of one member are walked while the next
-    // one's projection is still under way (two 11008 x 4096: 10 to 11 us one after the other, 13 together).
-    const bool together = static_cast<size_t>(all_k) * (MT < 4 ? MT : 4) * 4u <= 32u * 1024u &&
-                          p.n_tasks <= 2u * static_cast<uint32_t>(ctx->sm_count);
+    // Together as long as the slices leave room for two CTAs on an SM, and only
+    //  * where every CTA has at most one projection task: where they have more, the rows of one member are
+    //    walked while the next one's projection is still under way (two 11008 x 4096: 10 to 11 us one
+    //    after the other, 13 together);
+    //  * where a thread's words of the hand-over are one round of sixteen polls: with more, words that
+    //    are there wait for the last member's (two 1082 x 2100 of 256 atoms at four tokens, 24 words: 14.8 us
+    //    one after the other, 16.3 together; two 300-atom members of width 4572, 50 words: 18.3 and 22.8;
+    //    three 8601 x 876 of 512 atoms at two tokens, 12 words: 14.5 and 11.3).
+    const uint32_t tokens = MT < 4 ? MT : 4;
+    const bool together = p.n_seg > 1u && static_cast<size_t>(all_k) * tokens * 4u <= 32u * 1024u &&
+                          p.n_tasks <= 2u * static_cast<uint32_t>(ctx->sm_count) &&
+                          (all_k * tokens + kThreads - 1u) / kThreads * p.nsplit <= 16u;
     const uint32_t dx_atoms = together ? all_k : max_k;
-    plan.dxs_segs = together ? p.n_seg : 1u;
+    auto kern = together ? hsdr_gemv_fused_kernel<MT, A, U, true> : hsdr_gemv_fused_kernel<MT, A, U, false>;
     for (uint32_t i = 0; i < kMaxFusedGroup; ++i) plan.k_off[i + 1] = plan.k_off[i] + (i < p.n_seg ? p.seg[i].K : 0u);
     auto plan_for = [&](uint32_t gather_ctas) {
         size_t off = static_cast<size_t>(MT) * plan.xcols * 4u;
