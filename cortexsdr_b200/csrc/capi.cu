@@ -36,6 +36,35 @@ void DeviceBuffer::release_data() {
     bytes = 0;
 }
 
+void Built::record(cudaStream_t stream) {
+    if (!done) CSDR_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+    CSDR_CUDA(cudaEventRecord(done, stream));
+    pending = true;
+}
+
+bool Built::read_ahead(const csdr_context* ctx) {
+    if (!pending) return true;
+    cudaError_t e;
+    if (ctx->capturing()) {
+        // the build is no part of what is captured: it is waited for here, which a capture allows only in
+        // the relaxed mode
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        CSDR_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        e = cudaEventSynchronize(done);
+        CSDR_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    } else {
+        e = cudaEventQuery(done);
+    }
+    if (e == cudaErrorNotReady) {
+        (void)cudaGetLastError();
+        CSDR_CUDA(cudaStreamWaitEvent(ctx->stream, done, 0));
+        return false;
+    }
+    CSDR_CUDA(e);
+    pending = false;
+    return true;
+}
+
 Geometry make_geometry(const csdr_payload_info& v) {
     Geometry g;
     g.rows = v.rows;

@@ -15,6 +15,8 @@
 #include "host/format.hpp"
 #include "host/host_copy.hpp"
 
+struct csdr_context;
+
 namespace csdr {
 
 void set_last_error(const std::string& msg);
@@ -49,6 +51,17 @@ int guard(F&& f) {
                                                    cudaGetErrorString(_e));               \
     } while (0)
 
+// What a launch builds on first use and later launches read ahead of their dependency wait: safe once
+// the build is known to be complete, on whatever stream.
+struct Built {
+    cudaEvent_t done = nullptr;      // recorded behind the build
+    bool pending = false;            // not known to have completed
+    void record(cudaStream_t stream);
+    // False: the stream now waits for the build, and this launch must not start ahead of it.
+    bool read_ahead(const csdr_context* ctx);
+    ~Built() { if (done) cudaEventDestroy(done); }
+};
+
 // Device buffer with shared ownership (dictionaries are shared between a segment,
 // its row shards and, in a .hsda, every segment of a role).
 struct DeviceBuffer {
@@ -57,6 +70,7 @@ struct DeviceBuffer {
     int device = 0;
     // Derived data cached beside the buffer and freed with it (a dictionary's bf16 planes).
     std::shared_ptr<void> aux;
+    Built built;
     // A dictionary's atoms re-laid in the blocks the list kernel's loader fetches (gemv_queue.cu).
     std::shared_ptr<DeviceBuffer> stage_blocks;
     DeviceBuffer(size_t n, int dev);

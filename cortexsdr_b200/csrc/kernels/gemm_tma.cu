@@ -627,7 +627,7 @@ hsdr_tile_project_mma_kernel(const __grid_constant__ CUtensorMap map_hi, const _
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     __syncthreads();
-    // weight blocks of this CTA's walk, nobody else's output: read ahead
+    // weight blocks of this CTA's walk, complete before the launch: read ahead
     uint32_t l_stage = 0, l_tile = blockIdx.x, l_kb = 0;
     auto load = [&]() {
         const uint32_t bar = smem_u32(&full_bar[l_stage]), dst = smem_u32(ring + l_stage * stage_bytes);
@@ -827,6 +827,7 @@ std::shared_ptr<Planes> planes_for(csdr_context* ctx, const csdr_segment* seg) {
             static_cast<const float4*>(atoms->ptr), reinterpret_cast<uint2*>(hi), reinterpret_cast<uint2*>(lo), n / 4u);
         ls.done("split_planes_kernel");
     }
+    pl->buf->built.record(ctx->stream);
     pl->map_hi = make_map(hi, g.n_atoms, g.cols, kTileM);
     pl->map_lo = make_map(lo, g.n_atoms, g.cols, kTileM);
     atoms->aux = pl;
@@ -879,9 +880,11 @@ void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uin
     Params p{};
     p.n_seg = n_seg;
     uint32_t atom_tiles = 0;
+    bool ahead = true;      // the planes are complete: their loads may go ahead of the launch before
     for (uint32_t i = 0; i < n_seg; ++i) {
         if (segs[i]->g.cols != cols) throw Error(CSDR_ERR_GEOMETRY, "projection group: members differ in columns");
         auto weights = planes_for(ctx, segs[i]);
+        if (!weights->buf->built.read_ahead(ctx)) ahead = false;
         maps.hi[i] = weights->map_hi;
         maps.lo[i] = weights->map_lo;
         p.tile_begin[i] = atom_tiles;
@@ -927,7 +930,7 @@ void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uin
     attr[0].val.clusterDim.x = 1;
     attr[0].val.clusterDim.y = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
+    attr[1].val.programmaticStreamSerializationAllowed = ctx->pdl && ahead ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
 
@@ -1050,7 +1053,7 @@ void launch_tile_project(csdr_context* ctx, const csdr_segment* tile_view, const
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
+    attr[0].val.programmaticStreamSerializationAllowed = planes->buf->built.read_ahead(ctx) && ctx->pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     LaunchScope ls(ctx, KC_GEMM);

@@ -754,7 +754,7 @@ void stage_activations(csdr_context* ctx, const QueueItem* items, uint32_t n, QT
 
 // Built on a dictionary's first use by the list kernel and kept with it (as many bytes again as the
 // atoms): not inside a stream capture, like every first use that allocates.
-const DeviceBuffer* stage_blocks_of(csdr_context* ctx, const csdr_segment* seg) {
+DeviceBuffer* stage_blocks_of(csdr_context* ctx, const csdr_segment* seg) {
     DeviceBuffer* atoms = seg->atoms.get();
     if (!atoms->stage_blocks) {
         const Geometry& g = seg->g;
@@ -764,13 +764,14 @@ const DeviceBuffer* stage_blocks_of(csdr_context* ctx, const csdr_segment* seg) 
         stage_blocks_kernel<<<static_cast<unsigned>(std::min<size_t>((n + 255) / 256, static_cast<size_t>(ctx->sm_count) * 16)), 256, 0, ctx->stream>>>(
             static_cast<const float*>(atoms->ptr), g.n_atoms, g.cols, static_cast<float*>(blocks->ptr));
         ls.done("stage_blocks_kernel");
+        blocks->built.record(ctx->stream);
         atoms->stage_blocks = blocks;
     }
     return atoms->stage_blocks.get();
 }
 
 template <int MT>
-void launch_t(csdr_context* ctx, QParams& p, uint32_t max_k, uint32_t max_code_bytes) {
+void launch_t(csdr_context* ctx, QParams& p, uint32_t max_k, uint32_t max_code_bytes, bool ahead) {
     auto kern = hsdr_gemv_queue_kernel<MT>;
     p.stage_bytes = stage_bytes_for(MT);
     p.codes_bytes = codes_bytes_for(max_code_bytes);
@@ -789,7 +790,7 @@ void launch_t(csdr_context* ctx, QParams& p, uint32_t max_k, uint32_t max_code_b
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
+    attr[0].val.programmaticStreamSerializationAllowed = ctx->pdl && ahead ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     LaunchScope ls(ctx, KC_GEMV_QUEUE);
@@ -868,11 +869,14 @@ void launch_gemv_queue(csdr_context* ctx, const QueueItem* items, uint32_t n) {
         u64* scratch = static_cast<u64*>(ctx->scratch_get(6, std::max<size_t>(words * 8u, 4u << 20)));
         p.sumsq = scratch;
         p.dx = scratch + sumsq_words;
+        bool ahead = true;      // the blocks are complete: their loads may go ahead of the launch before
         for (uint32_t i = 0; i < cnt; ++i) {
             const QueueItem& it = items[i0 + i];
             const Geometry& g = it.seg->g;
             QTask& t = p.task[i];
-            t.D = static_cast<const float*>(stage_blocks_of(ctx, it.seg)->ptr);
+            DeviceBuffer* const blocks = stage_blocks_of(ctx, it.seg);
+            if (!blocks->built.read_ahead(ctx)) ahead = false;
+            t.D = static_cast<const float*>(blocks->ptr);
             t.codes = it.seg->codes_ptr();
             t.scales = static_cast<const float*>(it.seg->scales->ptr);
             t.x = it.x;
@@ -915,9 +919,9 @@ void launch_gemv_queue(csdr_context* ctx, const QueueItem* items, uint32_t n) {
         p.spin_barrier = ctx->spin_limit_barrier;
         p.trace = ctx->gemv_trace ? static_cast<unsigned long long*>(ctx->gemv_trace->ptr) : nullptr;
         switch (mt) {
-            case 1: launch_t<1>(ctx, p, max_k, max_code_bytes); break;
-            case 2: launch_t<2>(ctx, p, max_k, max_code_bytes); break;
-            default: launch_t<4>(ctx, p, max_k, max_code_bytes); break;
+            case 1: launch_t<1>(ctx, p, max_k, max_code_bytes, ahead); break;
+            case 2: launch_t<2>(ctx, p, max_k, max_code_bytes, ahead); break;
+            default: launch_t<4>(ctx, p, max_k, max_code_bytes, ahead); break;
         }
     }
 }
