@@ -117,52 +117,51 @@ __device__ __forceinline__ uint32_t entry(uint32_t row, uint32_t atom, float v) 
     return (off >> 1) << 16 | *reinterpret_cast<const unsigned short*>(&b);
 }
 
-// Code stream -> entries sorted by (row tile, atom block), codes that name an atom twice added up.
-// CTA = row tile, thread = row. starts[tile * (blocks + 1) + block]: first entry of a block's list
-// (the last one: its end); a tile's lists lie in its own rows-x-slots piece of `entries`.
-__global__ void __launch_bounds__(kRowsTile)
+// Code stream -> entries sorted by (row tile, atom block), codes that name an atom twice added up (exactly:
+// see exact_in_bf16). CTA = row tile, a thread takes every 1024th code; inside a block's list the order is
+// whatever the counters gave, as every entry has a place of its own in the block.
+// starts[tile * (blocks + 1) + block]: first entry of a block's list (the last one: its end); a tile's
+// lists lie in its own rows-x-slots piece of `entries`.
+constexpr uint32_t kEntryThreads = 1024, kCodesEach = kRowsTile * kMaxSlots / kEntryThreads;
+__global__ void __launch_bounds__(kEntryThreads)
 coefficient_entries_kernel(const uint16_t* __restrict__ codes, const float* __restrict__ scales, uint32_t R, uint32_t S, uint32_t k,
                            uint32_t n_blocks, uint32_t* __restrict__ entries, uint32_t* __restrict__ starts) {
-    __shared__ uint32_t count_s[kMaxBlocks][kRowsTile];
-    __shared__ uint32_t start_s[kMaxBlocks + 1];
-    const uint32_t slots = S * k, r = threadIdx.x, row = blockIdx.x * kRowsTile + r;
-    uint32_t atom[kMaxSlots];
-    float coef[kMaxSlots];
-    uint32_t n = 0;
-    for (uint32_t s = 0; row < R && s < slots; ++s) {
-        const uint32_t code = codes[static_cast<size_t>(row) * slots + s], a = code & 0x7FFFu;
-        const float g = (code & 0x8000u) ? -scales[s / k] : scales[s / k];
-        uint32_t i = 0;
-        while (i < n && atom[i] != a) ++i;
-        if (i == n) {
-            atom[n] = a;
-            coef[n++] = 0.0f;
-        }
-        coef[i] += g;
-    }
-    for (uint32_t b = 0; b < n_blocks; ++b) count_s[b][r] = 0;
-    for (uint32_t i = 0; i < n; ++i) ++count_s[atom[i] / kAtomBlock][r];
+    __shared__ uint16_t code_s[kRowsTile * kMaxSlots];
+    __shared__ float scale_s[kMaxSlots];
+    __shared__ uint32_t count_s[kMaxBlocks], start_s[kMaxBlocks + 1];
+    const uint32_t slots = S * k, tid = threadIdx.x, row0 = blockIdx.x * kRowsTile;
+    const uint32_t n = min(kRowsTile, R - row0) * slots;
+    for (uint32_t i = tid; i < n; i += kEntryThreads) code_s[i] = codes[static_cast<size_t>(row0) * slots + i];
+    if (tid < S) scale_s[tid] = scales[tid];
+    if (tid < n_blocks) count_s[tid] = 0;
     __syncthreads();
-    if (r < n_blocks) {       // a block's rows one behind the other
-        uint32_t at = 0;
-        for (uint32_t q = 0; q < kRowsTile; ++q) {
-            const uint32_t c = count_s[r][q];
-            count_s[r][q] = at;
-            at += c;
-        }
-        start_s[r + 1u] = at;
+    uint32_t held[kCodesEach], place[kCodesEach];      // an entry; its block and index there (none: all ones)
+#pragma unroll
+    for (uint32_t j = 0; j < kCodesEach; ++j) {
+        place[j] = 0xFFFFFFFFu;
+        const uint32_t i = tid + j * kEntryThreads;
+        if (i >= n) continue;
+        const uint32_t r = i / slots, s = i - r * slots, a = code_s[i] & 0x7FFFu;
+        const uint16_t* row = code_s + r * slots;
+        bool first = true;
+        for (uint32_t q = 0; q < s; ++q) first = first && (row[q] & 0x7FFFu) != a;
+        if (!first) continue;                          // the first code that names an atom stands for all
+        float coef = 0.0f;
+        for (uint32_t q = s; q < slots; ++q)
+            if ((row[q] & 0x7FFFu) == a) coef += (row[q] & 0x8000u) ? -scale_s[q / k] : scale_s[q / k];
+        held[j] = entry(r, a, coef);
+        place[j] = (a / kAtomBlock) << 16 | atomicAdd(&count_s[a / kAtomBlock], 1u);
     }
     __syncthreads();
-    if (r == 0) {
-        start_s[0] = blockIdx.x * kRowsTile * slots;
-        for (uint32_t b = 0; b < n_blocks; ++b) start_s[b + 1u] += start_s[b];
+    if (tid == 0) {
+        start_s[0] = row0 * slots;
+        for (uint32_t b = 0; b < n_blocks; ++b) start_s[b + 1u] = start_s[b] + count_s[b];
     }
     __syncthreads();
-    if (r <= n_blocks) starts[blockIdx.x * (n_blocks + 1u) + r] = start_s[r];
-    for (uint32_t i = 0; i < n; ++i) {
-        const uint32_t b = atom[i] / kAtomBlock;
-        entries[start_s[b] + count_s[b][r]++] = entry(r, atom[i], coef[i]);
-    }
+    if (tid <= n_blocks) starts[blockIdx.x * (n_blocks + 1u) + tid] = start_s[tid];
+#pragma unroll
+    for (uint32_t j = 0; j < kCodesEach; ++j)
+        if (place[j] != 0xFFFFFFFFu) entries[start_s[place[j] >> 16] + (place[j] & 0xFFFFu)] = held[j];
 }
 
 struct GatherMmaParams {
@@ -484,31 +483,31 @@ EncodeFn encode_fn() {
     return fn;
 }
 
-// The segment's entries, built on its first wide product and kept with it (4 bytes a code).
-const uint32_t* entries_of(csdr_context* ctx, const csdr_segment* seg, const uint32_t** starts) {
+// The segment's entries, built on its first wide product and kept with it (4 bytes a code). False where
+// they are missing: under capture, or without room.
+bool build_entries(csdr_context* ctx, const csdr_segment* seg) {
+    if (seg->coefficients) return true;
+    if (ctx->capturing()) return false;
     const Geometry& g = seg->g;
     const uint32_t tiles = (g.rows + kRowsTile - 1u) / kRowsTile, nb = g.n_atoms / kAtomBlock;
     const size_t n_entries = static_cast<size_t>(tiles) * kRowsTile * g.slots();
-    if (!seg->coefficients) {
-        auto buf = std::make_shared<DeviceBuffer>((n_entries + static_cast<size_t>(tiles) * (nb + 1u)) * 4u, ctx->device);
-        uint32_t* e = static_cast<uint32_t*>(buf->ptr);
-        LaunchScope ls(ctx, KC_GATHER);
-        coefficient_entries_kernel<<<tiles, kRowsTile, 0, ctx->stream>>>(seg->codes_ptr(), static_cast<const float*>(seg->scales->ptr), g.rows,
-                                                                       g.n_stages, g.k, nb, e, e + n_entries);
-        ls.done("coefficient_entries_kernel");
-        CSDR_CUDA(cudaStreamSynchronize(ctx->stream));   // later launches read them ahead of their dependency wait
-        seg->coefficients = buf;
-    }
-    const uint32_t* e = static_cast<const uint32_t*>(seg->coefficients->ptr);
-    *starts = e + n_entries;
-    return e;
+    const DevPtr buf = ctx->try_keep((n_entries + static_cast<size_t>(tiles) * (nb + 1u)) * 4u);
+    if (!buf) return false;
+    uint32_t* e = static_cast<uint32_t*>(buf->ptr);
+    LaunchScope ls(ctx, KC_GATHER);
+    coefficient_entries_kernel<<<tiles, kEntryThreads, 0, ctx->stream>>>(seg->codes_ptr(), static_cast<const float*>(seg->scales->ptr), g.rows,
+                                                                         g.n_stages, g.k, nb, e, e + n_entries);
+    ls.done("coefficient_entries_kernel");
+    buf->built.record(ctx->stream);
+    seg->coefficients = buf;
+    return true;
 }
 
 size_t gather_mma_smem(uint32_t n_atoms) { return 3u * static_cast<size_t>(n_atoms) * 128u + 2u * kABytes + 1024u; }
 
 }  // namespace
 
-bool gather_mma_supported(const csdr_context* ctx, const csdr_segment* seg, size_t batch) {
+bool gather_mma_ready(csdr_context* ctx, const csdr_segment* seg, size_t batch) {
     const Geometry& g = seg->g;
     if (!ctx->gather_mma || !ctx->tensor_cores || !ctx->tma || !encode_fn()) return false;
     if (!g.row_tiles() || g.n_atoms % (2u * kAtomBlock) || g.n_atoms > kMaxBlocks * kAtomBlock || g.slots() > kMaxSlots) return false;
@@ -524,14 +523,15 @@ bool gather_mma_supported(const csdr_context* ctx, const csdr_segment* seg, size
         return false;
     if (static_cast<uint64_t>((g.rows + kRowsTile - 1u) / kRowsTile) * kRowsTile * g.slots() > 0x7FFFFFFFull) return false;
     if (gather_mma_smem(g.n_atoms) + 1024u > ctx->smem_optin || !exact_in_bf16(seg->scales_host, g.k)) return false;
-    return seg->coefficients || !ctx->capturing();   // the entries are built on first use
+    return build_entries(ctx, seg);
 }
 
 void launch_gather_mma(csdr_context* ctx, const csdr_segment* seg, const DxPlanes& dx, uint32_t M, const YView& y, const float* residual,
                        const TokenScale& ts) {
     const Geometry& g = seg->g;
     GatherMmaParams p{};
-    p.entries = entries_of(ctx, seg, &p.starts);
+    p.entries = static_cast<const uint32_t*>(seg->coefficients->ptr);
+    p.starts = p.entries + static_cast<size_t>((g.rows + kRowsTile - 1u) / kRowsTile) * kRowsTile * g.slots();
     p.codes = seg->codes_ptr();
     p.scales = static_cast<const float*>(seg->scales->ptr);
     p.planes = dx.p;
@@ -565,7 +565,7 @@ void launch_gather_mma(csdr_context* ctx, const csdr_segment* seg, const DxPlane
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
+    attr[0].val.programmaticStreamSerializationAllowed = seg->coefficients->built.read_ahead(ctx) && ctx->pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     LaunchScope ls(ctx, KC_GATHER);

@@ -992,7 +992,7 @@ WideDx launch_wide_project(csdr_context* ctx, const csdr_segment* const* segs, u
     size_t total_atoms = 0;
     for (uint32_t i = 0; i < n; ++i) total_atoms += segs[i]->g.n_atoms;
     bool as_planes = !fp32_dx && M > 16u && !(xch && xch->ranks > 1u);
-    for (uint32_t i = 0; i < n; ++i) as_planes = as_planes && gather_mma_supported(ctx, segs[i], M);
+    for (uint32_t i = 0; i < n; ++i) as_planes = as_planes && gather_mma_ready(ctx, segs[i], M);
     if (as_planes) {
         w.stride = (M + 7u) & ~7u;
         __nv_bfloat16* at = static_cast<__nv_bfloat16*>(ctx->scratch_get(0, total_atoms * w.stride * 6u));
@@ -1139,7 +1139,7 @@ void launch_matmul_tcgen05(csdr_context* ctx, const csdr_segment* seg, const Mat
     const uint32_t kb_per_split = (n_kb + n_split - 1u) / n_split;
     n_split = (n_kb + kb_per_split - 1u) / kb_per_split;
 
-    if (M > 16u && g.n_stages <= 64u && dx_tma_supported(ctx, seg, a.batch) && gather_mma_supported(ctx, seg, M)) {
+    if (M > 16u && g.n_stages <= 64u && dx_tma_supported(ctx, seg, a.batch) && gather_mma_ready(ctx, seg, M)) {
         const WideOut out{a.y, a.bias, nullptr};
         launch_matmul_wide_group(ctx, &seg, 1, make_x_planes(ctx, a.x, a.x_dtype, a.x_layout, M, g.cols), M, &out, a.y_layout);
         return;

@@ -784,12 +784,13 @@ void launch_matmul(csdr_context* ctx, const csdr_segment* seg, const MatmulArgs&
         if (!seg->dense_f32 && !ctx->capturing()) {
             if (const DevPtr w = ctx->try_keep(static_cast<size_t>(g.rows) * g.cols * 4u)) {
                 launch_decode_rows(ctx, seg, nullptr, g.rows, static_cast<float*>(w->ptr));
-                CSDR_CUDA(cudaStreamSynchronize(ctx->stream));
+                w->built.record(ctx->stream);
                 seg->dense_f32 = w;
             }
         }
         if (seg->dense_f32) {
-            launch_dense_matmul(ctx, static_cast<const float*>(seg->dense_f32->ptr), g.rows, g.cols, a, false);
+            const bool fresh = !seg->dense_f32->built.read_ahead(ctx);
+            launch_dense_matmul(ctx, static_cast<const float*>(seg->dense_f32->ptr), g.rows, g.cols, a, fresh);
             return;
         }
     }
