@@ -509,13 +509,11 @@ void launch_t(csdr_context* ctx, FusedParams& p, uint32_t max_k, bool pdl) {
     //    one after the other, 16.3 together; two 300-atom members of width 4572, 50 words: 18.3 and 22.8;
     //    three 8601 x 876 of 512 atoms at two tokens, 12 words: 14.5 and 11.3).
     const uint32_t tokens = MT < 4 ? MT : 4;
-    const bool together = p.n_seg > 1u && static_cast<size_t>(all_k) * tokens * 4u <= 32u * 1024u &&
+    bool together = p.n_seg > 1u && static_cast<size_t>(all_k) * tokens * 4u <= 32u * 1024u &&
                           p.n_tasks <= 2u * static_cast<uint32_t>(ctx->sm_count) &&
                           (all_k * tokens + kThreads - 1u) / kThreads * p.nsplit <= 16u;
-    const uint32_t dx_atoms = together ? all_k : max_k;
-    auto kern = together ? hsdr_gemv_fused_kernel<MT, A, U, true> : hsdr_gemv_fused_kernel<MT, A, U, false>;
     for (uint32_t i = 0; i < kMaxFusedGroup; ++i) plan.k_off[i + 1] = plan.k_off[i] + (i < p.n_seg ? p.seg[i].K : 0u);
-    auto plan_for = [&](uint32_t gather_ctas) {
+    auto plan_for = [&](uint32_t gather_ctas, uint32_t dx_atoms) {
         size_t off = static_cast<size_t>(MT) * plan.xcols * 4u;
         for (uint32_t i = 0; i < p.n_seg; ++i) {
             const uint32_t chunks = std::max<uint32_t>(1u, gather_ctas / token_groups);
@@ -534,8 +532,15 @@ void launch_t(csdr_context* ctx, FusedParams& p, uint32_t max_k, bool pdl) {
         return off + (p.norm_w ? static_cast<size_t>(p.C) * 4u : 0u);
     };
     const uint32_t want_gather = p.gather_ctas;
-    const size_t smem = plan_for(std::min<uint32_t>(want_gather, static_cast<uint32_t>(ctx->sm_count)));
+    const uint32_t least = std::min<uint32_t>(want_gather, static_cast<uint32_t>(ctx->sm_count));
+    const size_t alone = plan_for(least, max_k), smem_all = plan_for(least, all_k);
+    //  * and where all slices fit, with as many CTAs on an SM as one slice at a time leaves room for (half
+    //    the opt-in size holds two, static shared memory and what the driver keeps included).
+    const size_t two = ctx->smem_optin / 2u - 2048u;
+    together = together && smem_all <= (alone <= two ? two : ctx->smem_optin);
+    const size_t smem = together ? smem_all : alone;
     if (smem > ctx->smem_optin) throw Error(CSDR_ERR_LIMIT, "fused GEMV: shared memory need exceeds the device limit");
+    auto kern = together ? hsdr_gemv_fused_kernel<MT, A, U, true> : hsdr_gemv_fused_kernel<MT, A, U, false>;
     ctx->opt_in_smem(reinterpret_cast<const void*>(kern), smem);
     std::pair<size_t, int>& occ = ctx->occupancy[reinterpret_cast<const void*>(kern)];
     if (occ.second == 0 || occ.first != smem) {
@@ -549,7 +554,7 @@ void launch_t(csdr_context* ctx, FusedParams& p, uint32_t max_k, bool pdl) {
     // Every CTA must be resident for the barrier: at most what one otherwise idle GPU holds.
     const uint32_t grid = static_cast<uint32_t>(ctx->sm_count) * static_cast<uint32_t>(std::min(occ_cached, 2));
     p.gather_ctas = std::max(token_groups, std::min(want_gather, grid) / token_groups * token_groups);
-    plan_for(p.gather_ctas);  // never larger than the size computed above
+    plan_for(p.gather_ctas, together ? all_k : max_k);  // never larger than the size computed above
     // whole-x residency only pays when a CTA walks several column slabs (the folded normalisation
     // needs it regardless: every CTA sums the squares of the whole row)
     if (!p.norm_w && plan.xcols == p.C && p.n_tasks <= grid && p.slab < p.C) {
