@@ -528,6 +528,7 @@ void launch_t(csdr_context* ctx, FusedParams& p, uint32_t max_k, bool pdl) {
         }
         plan.dxs_off = static_cast<uint32_t>(off);
         off += static_cast<size_t>(dx_atoms) * (MT < 4 ? MT : 4) * 4u;
+        off = (off + 15u) & ~static_cast<size_t>(15);      // 16-byte copies, behind slices of any size
         plan.normw_off = static_cast<uint32_t>(off);
         return off + (p.norm_w ? static_cast<size_t>(p.C) * 4u : 0u);
     };
