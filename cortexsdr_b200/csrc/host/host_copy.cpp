@@ -12,13 +12,14 @@ namespace {
 constexpr size_t kSlot = 512u << 10;      // bytes of a page-locked slot
 constexpr size_t kMaxWorkers = 8;
 
-bool page_locked(const void* p) {
+// Memory the driver knows nothing of. What it knows (page-locked, managed, device) is its to copy or to refuse.
+bool pageable(const void* p) {
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
-    return at.type == cudaMemoryTypeHost;
+    return at.type == cudaMemoryTypeUnregistered;
 }
 }  // namespace
 
@@ -140,7 +141,7 @@ void HostCopier::copy(void* dst, const void* src, size_t bytes, bool up) {
     if (!bytes) return;
     std::lock_guard<std::mutex> call(call_);
     // cudaStreamPerThread names another stream in every helper: its copies stay with the calling thread
-    if (bytes < kSmall || stream_ == cudaStreamPerThread || page_locked(up ? src : dst) || !start()) {
+    if (bytes < kSmall || stream_ == cudaStreamPerThread || !pageable(up ? src : dst) || !start()) {
         CSDR_CUDA(cudaMemcpyAsync(dst, src, bytes, up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, stream_));
         // a page-locked source is read behind the call's return: wait, as for a download
         CSDR_CUDA(cudaStreamSynchronize(stream_));

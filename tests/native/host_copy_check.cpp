@@ -15,6 +15,7 @@ namespace {
 std::mutex mu;
 std::set<std::thread::id> copied_from;
 size_t copied = 0;
+cudaMemoryType kind = cudaMemoryTypeUnregistered;      // of every host pointer
 }  // namespace
 
 extern "C" {
@@ -26,7 +27,7 @@ cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind
     return cudaSuccess;
 }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* at, const void*) {
-    at->type = cudaMemoryTypeUnregistered;
+    at->type = kind;
     return cudaSuccess;
 }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
@@ -71,6 +72,17 @@ int main() {
                 return 1;
             }
         }
+    // memory the driver knows is copied, or refused, by the driver
+    for (cudaMemoryType known : {cudaMemoryTypeHost, cudaMemoryTypeDevice, cudaMemoryTypeManaged}) {
+        kind = known;
+        csdr::HostCopier copier(0, own);
+        copied_from.clear();
+        copier.download(dst.data(), src.data(), src.size());
+        if (copied_from.size() != 1 || !copied_from.count(std::this_thread::get_id())) {
+            std::printf("memory of type %d was copied from %zu threads\n", static_cast<int>(known), copied_from.size());
+            return 1;
+        }
+    }
     std::printf("ok\n");
     return 0;
 }
