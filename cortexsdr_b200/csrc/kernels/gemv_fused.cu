@@ -132,11 +132,12 @@ struct SmemPlan {
 
 // Register budget: two launches must be able to sit on an SM together (two CTAs each), or the
 // next launch's weight prefetch cannot start before this one retires.
-// TOGETHER: the segments of a group are handed over and their rows walked together, with one barrier
-// between (a CTA has 16 rows of a 4864-row segment for its 256 threads: gate and up of 4864 x 896 7.5 us
-// against 8.4 one after the other). What places an element or a row among several costs a single product
-// 0.4 us of its 5.9 and is in this instance only.
-template <int MT, int A, int U, bool TOGETHER>
+// How the segments of a launch are gathered. kTogether: handed over and their rows walked together, with
+// one barrier between (a CTA has 16 rows of a 4864-row segment for its 256 threads: gate and up of 4864 x
+// 896 6.9 us against 8.4 in turn). What places an element or a row among several, and what it takes to
+// come back for the next segment, costs a single product up to 0.4 us of its 5.9: instances.
+enum class Walk { kOne, kInTurn, kTogether };
+template <int MT, int A, int U, Walk WALK>
 __global__ void __launch_bounds__(kThreads, (MT <= 4 ? 4 : 3))
 hsdr_gemv_fused_kernel(const __grid_constant__ FusedParams p, const __grid_constant__ SmemPlan plan) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -208,7 +209,7 @@ hsdr_gemv_fused_kernel(const __grid_constant__ FusedParams p, const __grid_const
             const FusedSeg& sg = p.seg[si];
             const uint32_t row0 = rchunk * sg.rows_per_cta;
             rows_before += row0 < sg.R ? min(sg.rows_per_cta, sg.R - row0) : 0u;
-            if (TOGETHER && tid == 0) r_off_s[si + 1u] = rows_before;
+            if (WALK == Walk::kTogether && tid == 0) r_off_s[si + 1u] = rows_before;
             if (row0 < sg.R) {
                 const uint32_t rows_here = min(sg.rows_per_cta, sg.R - row0);
                 const uint32_t slots = sg.S * sg.k;
@@ -427,7 +428,7 @@ hsdr_gemv_fused_kernel(const __grid_constant__ FusedParams p, const __grid_const
         if (live) {
             if (p.norm_w) accr *= inv_s[tok];
             if (sg.y.bias) accr += bias_v;
-            if (p.swiglu && si == 1u) {
+            if (WALK != Walk::kOne && p.swiglu && si == 1u) {
                 // silu_mul (api/cortex_sdk.cpp:1245-1256); this thread wrote the gate row itself
                 const float gv = p.seg[0].y.y[yi];
                 accr = (gv * (1.0f / (1.0f + expf(-gv)))) * accr;
@@ -442,7 +443,7 @@ hsdr_gemv_fused_kernel(const __grid_constant__ FusedParams p, const __grid_const
     };
     auto scales_of = [&](uint32_t si) { return reinterpret_cast<const float*>(smem_raw + plan.scales_off[si]); };
     constexpr uint32_t RP = kThreads / MTG;
-    if constexpr (TOGETHER) {
+    if constexpr (WALK == Walk::kTogether) {
         const uint32_t n_rows = r_off_s[p.n_seg];
         if (n_rows)
             hand_over(plan.k_off[p.n_seg], [&](uint32_t sp, uint32_t a) {
@@ -466,7 +467,8 @@ hsdr_gemv_fused_kernel(const __grid_constant__ FusedParams p, const __grid_const
             }
         }
     } else {
-        for (uint32_t si = 0; si < p.n_seg; ++si) {
+        const uint32_t n_seg = WALK == Walk::kOne ? 1u : p.n_seg;
+        for (uint32_t si = 0; si < n_seg; ++si) {
             const FusedSeg& sg = p.seg[si];
             const uint32_t row0 = rchunk * sg.rows_per_cta;
             if (row0 < sg.R) {
@@ -480,7 +482,7 @@ hsdr_gemv_fused_kernel(const __grid_constant__ FusedParams p, const __grid_const
                 const uint16_t* cs = codes_of(sg, si);
                 for (uint32_t rl = tid / MTG; rl < rows_here; rl += RP) finish(sg, si, row0 + rl, cs + rl * slots, scales_of(si), dxs);
             }
-            if (si + 1u < p.n_seg) __syncthreads();  // dxs is rewritten for the next segment
+            if (si + 1u < n_seg) __syncthreads();  // dxs is rewritten for the next segment
         }
     }
     if (late) atomicExch(p.status, 1);
@@ -541,7 +543,8 @@ void launch_t(csdr_context* ctx, FusedParams& p, uint32_t max_k, bool pdl) {
     together = together && smem_all <= (alone <= two ? two : ctx->smem_optin);
     const size_t smem = together ? smem_all : alone;
     if (smem > ctx->smem_optin) throw Error(CSDR_ERR_LIMIT, "fused GEMV: shared memory need exceeds the device limit");
-    auto kern = together ? hsdr_gemv_fused_kernel<MT, A, U, true> : hsdr_gemv_fused_kernel<MT, A, U, false>;
+    auto kern = together ? hsdr_gemv_fused_kernel<MT, A, U, Walk::kTogether>
+                : p.n_seg > 1u ? hsdr_gemv_fused_kernel<MT, A, U, Walk::kInTurn> : hsdr_gemv_fused_kernel<MT, A, U, Walk::kOne>;
     ctx->opt_in_smem(reinterpret_cast<const void*>(kern), smem);
     std::pair<size_t, int>& occ = ctx->occupancy[reinterpret_cast<const void*>(kern)];
     if (occ.second == 0 || occ.first != smem) {
