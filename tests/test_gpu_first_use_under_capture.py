@@ -14,12 +14,15 @@ pytestmark = pytest.mark.gpu
     (700, 512, 0, 64, 300),      # planes built by a smaller batch; the gather's entries are not
     (1500, 1000, 128, 0, 2),     # ragged tiles: no rebuilt weight yet
 ])
-def test_first_use_under_capture(oracle, rows, cols, tile, warm, m):
+def test_first_use_under_capture(oracle, monkeypatch, rows, cols, tile, warm, m):
     def payload(r, atoms, **kw):
         return synth.hsdr_payload(r, cols, tile_rows=tile or 1, tile_cols=tile or cols, n_atoms=atoms, k=8, seed=r, **kw)
 
     st = torch.cuda.Stream()
     ctx = cs.Context(0, st.cuda_stream)
+    monkeypatch.setenv("CSDR_GATHER_MMA", "0")
+    monkeypatch.setenv("CSDR_CACHE_2D", "0")
+    plain = cs.Context(0, st.cuda_stream)              # never builds what the captured call would
     pay = payload(rows, 128)
     seg = cs.Segment.from_payload(pay, ctx)
     # another segment that takes the fallback form anyway, so that the scratch has grown: stage scales
@@ -46,6 +49,15 @@ def test_first_use_under_capture(oracle, rows, cols, tile, warm, m):
     want = x.double().cpu().numpy() @ oracle.decompress(pay).astype(np.float64).T
     # two bf16 pieces of every operand in the first case, fp32 in the second
     assert np.linalg.norm(y.double().cpu().numpy() - want) <= 2e-5 * np.linalg.norm(want)
+    # the form that needs nothing built, to the bit; the call outside the capture takes the other one
+    bare = cs.Segment.from_payload(pay, plain)
+    y_plain, y_later = torch.zeros_like(y), torch.zeros_like(y)
+    call(bare, m, y_plain)
+    call(seg, m, y_later)
+    plain.synchronize()
+    ctx.synchronize()
+    assert torch.equal(y, y_plain) and not torch.equal(y, y_later)
+    bare.close()
     del g
     seg.close()
     other.close()

@@ -25,23 +25,30 @@ def run(monkeypatch, on, pays, x, dtype, token, bias):
     bd = torch.from_numpy(bias).cuda() if bias is not None else None
     code = cs.DTYPE_BF16 if dtype == "bf16" else cs.DTYPE_F32
     torch.cuda.synchronize()
+    counts = [ctx.launch_count]
     for _ in range(2):
         if len(segs) > 1:
             cs.Segment.matmul_group_device(segs, xin.data_ptr(), code, layout, m, [y.data_ptr() for y in ys], layout)
         else:
             segs[0].matmul_device(xin.data_ptr(), code, layout, m, ys[0].data_ptr(), layout, bd.data_ptr() if bd is not None else 0)
+        counts.append(ctx.launch_count)
     ctx.synchronize()
+    built = counts[1] - counts[0] - (counts[2] - counts[1])        # launches only the first call had
     out = [(y if token else y.t()).double().cpu().numpy() for y in ys]
     xd = t.double().cpu().numpy()
     for s in segs:
         s.close()
     ctx.close()
-    return out, xd
+    return out, xd, built
 
 
-def check(oracle, monkeypatch, pays, x, dtype, token, bias=None):
-    got, xd = run(monkeypatch, "1", pays, x, dtype, token, bias)
-    look, _ = run(monkeypatch, "0", pays, x, dtype, token, bias)
+def check(oracle, monkeypatch, pays, x, dtype, token, bias=None, taken=True):
+    """taken: the products go to the tensor cores (their entries are built, a launch a segment, and their
+    sums have another order than the lookups'); else both runs are the lookups'."""
+    got, xd, built = run(monkeypatch, "1", pays, x, dtype, token, bias)
+    look, _, planes = run(monkeypatch, "0", pays, x, dtype, token, bias)
+    assert built - planes == (len(pays) if taken else 0)
+    assert taken or all(np.array_equal(g, l) for g, l in zip(got, look))
     for g, l, pay in zip(got, look, pays):
         want = xd @ oracle.decompress(pay).astype(np.float64).T + (0 if bias is None else bias)
         # the same 24-bit projection, at most 64 exact terms in fp32: 64 * 2^-24 at the very most
@@ -76,7 +83,7 @@ def test_gather_products_of_a_group(oracle, monkeypatch):
 def test_other_stage_scales(oracle, monkeypatch, decay):
     pay = synth.hsdr_payload(200, 128, n_atoms=128, k=8, decay=decay, seed=4)
     x = np.random.default_rng(1).normal(0, 1, (70, 128)).astype(np.float32)
-    check(oracle, monkeypatch, [pay], x, "f32", True)
+    check(oracle, monkeypatch, [pay], x, "f32", True, taken=False)
 
 
 @pytest.mark.parametrize("token", [False, True])
@@ -95,8 +102,8 @@ def test_values_that_are_not_finite_stay_in_the_rows_that_name_them(monkeypatch,
     x[70, :big] = 1                                    # finite in fp32, past bf16's rounding
     x[71, 0] = 64                                      # past fp32
     x[140, 50] = np.nan
-    got, _ = run(monkeypatch, "1", [bytes(pay)], x, "f32", token, None)
-    look, _ = run(monkeypatch, "0", [bytes(pay)], x, "f32", token, None)
+    got, _, _ = run(monkeypatch, "1", [bytes(pay)], x, "f32", token, None)
+    look, _, _ = run(monkeypatch, "0", [bytes(pay)], x, "f32", token, None)
     codes = np.frombuffer(bytes(pay), np.uint16, rows * 24, 36 + 4 * 3 + 4 * atoms * cols).reshape(rows, 24) & 0x7FFF
     clean = ~np.isin(codes, (7, 20, 21)).any(axis=1)
     assert 100 < clean.sum() < rows
