@@ -575,6 +575,10 @@ hsdr_dx_tma_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant
 // the MMA's layout, the ring of weight blocks runs on across row tiles, and two accumulators let the
 // epilogue of one tile (tensor memory lanes are rows, so a warp stores 128 contiguous bytes of a
 // token's row) overlap the products of the next. Same products in the same order as before.
+// The gather behind is not let in early (no griddepcontrol.launch_dependents), and shared memory keeps
+// this launch at one CTA an SM: CTAs of either kernel placed while the other's are there crowd the SMs
+// that have none (4864 x 1024 in 64 x 64 tiles, 8 tokens 33 us, let in after the dependency wait 39.5;
+// 5376 x 3328 in 16 x 16 tiles, 2 tokens 113, let in at once 196).
 constexpr uint32_t kTileStages = 5;
 
 struct TileProjectParams {
@@ -585,6 +589,7 @@ struct TileProjectParams {
     uint32_t n_tile, n_kb, stages;
     uint32_t x_has_lo;
     uint32_t tmem_cols;
+    uint32_t x_vec;          // activations token-major on 16-byte boundaries
     int* status;
     uint32_t spin;
 };
@@ -594,7 +599,6 @@ __global__ void __launch_bounds__(kThreads, 1)
 hsdr_tile_project_mma_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
                              const __grid_constant__ TileProjectParams p) {
     extern __shared__ __align__(1024) unsigned char tma_smem_raw[];
-    asm volatile("griddepcontrol.launch_dependents;");
     __shared__ __align__(8) unsigned long long full_bar[kTileStages], empty_bar[kTileStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int failed_s;
@@ -650,15 +654,30 @@ hsdr_tile_project_mma_kernel(const __grid_constant__ CUtensorMap map_hi, const _
         const uint32_t kb = i / (N * 8u), r = i - kb * N * 8u, t = r >> 3, u = r & 7u;
         const uint32_t tok = tok0 + t, c0 = kb * kBlockK + u * 8u;
         alignas(16) __nv_bfloat16 h[8], l[8];
+        alignas(16) float v[8] = {};
+        if (tok < p.n_tok && c0 < p.Tc) {      // Tc is a multiple of eight
+            const uint32_t b = tok / p.n_ct, c = (tok - b * p.n_ct) * p.Tc + c0;
+            if (p.x_vec) {
+                const size_t at = static_cast<size_t>(p.x.b0 + b) * p.x.C + c;
+                if (p.x_has_lo) {
+                    const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(p.x.x) + at);
+                    *reinterpret_cast<float4*>(v) = src[0];
+                    *reinterpret_cast<float4*>(v + 4) = src[1];
+                } else {
+                    const uint4 w = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.x.x) + at);
+                    const __nv_bfloat16* s = reinterpret_cast<const __nv_bfloat16*>(&w);
+#pragma unroll
+                    for (uint32_t e = 0; e < 8u; ++e) v[e] = __bfloat162float(s[e]);
+                }
+            } else {
+#pragma unroll
+                for (uint32_t e = 0; e < 8u; ++e) v[e] = load_x(p.x, c + e, b);
+            }
+        }
 #pragma unroll
         for (uint32_t e = 0; e < 8u; ++e) {
-            float v = 0.0f;
-            if (tok < p.n_tok && c0 + e < p.Tc) {
-                const uint32_t b = tok / p.n_ct, bc = tok - b * p.n_ct;
-                v = load_x(p.x, bc * p.Tc + c0 + e, b);
-            }
-            h[e] = __float2bfloat16_rn(v);
-            l[e] = __float2bfloat16_rn(v - __bfloat162float(h[e]));
+            h[e] = __float2bfloat16_rn(v[e]);
+            l[e] = __float2bfloat16_rn(v[e] - __bfloat162float(h[e]));
         }
         unsigned char* dst = xs + kb * x_planes * b_tile + (t >> 3) * 1024u + (t & 7u) * 128u + ((u ^ (t & 7u)) << 4);
         *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(h);
@@ -685,7 +704,7 @@ hsdr_tile_project_mma_kernel(const __grid_constant__ CUtensorMap map_hi, const _
         bool ok = true;
         uint32_t s = 0, parity = 0, at = ring_lo;
         for (uint32_t ti = 0; ti < mine && ok; ++ti) {
-            const uint32_t acc = ti & 1u, d = tmem_base + acc * N;
+            const uint32_t acc = ti & 1u, d = tmem_base + acc * (p.tmem_cols / 2u);
             if (ti >= 2u) ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&acc_empty[acc]), (ti / 2u - 1u) & 1u, p.spin));
             for (uint32_t kb = 0; kb < p.n_kb && ok; ++kb) {
                 ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&full_bar[s]), parity, p.spin) && !failed_s);
@@ -719,7 +738,7 @@ hsdr_tile_project_mma_kernel(const __grid_constant__ CUtensorMap map_hi, const _
             float* dst = p.out + static_cast<size_t>(tok0) * p.rows + (blockIdx.x + ti * gridDim.x) * kTileM + row;
             for (uint32_t ch = 0; ch < N / 16u; ++ch) {
                 uint32_t r[16];
-                const uint32_t taddr = tmem_base + acc * N + ((quad * 32u) << 16) + ch * 16u;
+                const uint32_t taddr = tmem_base + acc * (p.tmem_cols / 2u) + ((quad * 32u) << 16) + ch * 16u;
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
@@ -1010,14 +1029,22 @@ void launch_dx_tma_group(csdr_context* ctx, const csdr_segment* const* segs, uin
     ls.done("hsdr_dx_tma_kernel");
 }
 
+namespace {
+// Tokens of a tile: as few tiles of at most 128 as there can be, all of one size (in sixteens). The CTAs of
+// a tile that is mostly padding finish early and leave their SMs idle (768 x 1536 in 128 x 128 tiles, 12
+// tokens, 144 column tiles as 128 + 16: 68 us for the whole product, as 80 + 64 54; 62 before this kernel).
+uint32_t tile_project_tokens(uint32_t n_tok) {
+    const uint32_t tiles = (n_tok + 127u) / 128u;
+    return ((n_tok + tiles - 1u) / tiles + 15u) & ~15u;
+}
+}  // namespace
+
 // Shared memory beside the barriers: the activations of a token tile and the ring of weight blocks.
 // At least three stages must fit, else the plain projection computes the tile products.
 bool tile_project_supported(const csdr_context* ctx, const csdr_segment* tile_view, size_t n_tok, bool x_has_lo) {
     using namespace tma_detail;
     if (!dx_tma_supported(ctx, tile_view, n_tok) || n_tok == 0 || n_tok > 0x7FFFFFFFu) return false;
-    const uint32_t n_kb = (tile_view->g.cols + kBlockK - 1u) / kBlockK;
-    uint32_t N = 16;
-    while (N < 128u && N < n_tok) N <<= 1;
+    const uint32_t n_kb = (tile_view->g.cols + kBlockK - 1u) / kBlockK, N = tile_project_tokens(static_cast<uint32_t>(n_tok));
     return static_cast<size_t>(n_kb) * (x_has_lo ? 2u : 1u) * N * 128u + 3u * 2u * kATile + 4096u <= ctx->smem_optin;
 }
 
@@ -1032,22 +1059,23 @@ void launch_tile_project(csdr_context* ctx, const csdr_segment* tile_view, const
     p.Tc = g.cols;
     p.n_ct = n_ct;
     p.n_tok = x.M * n_ct;
-    p.n_tile = 16;
-    while (p.n_tile < 128u && p.n_tile < p.n_tok) p.n_tile <<= 1;
+    p.n_tile = tile_project_tokens(p.n_tok);
     p.n_kb = (g.cols + kBlockK - 1u) / kBlockK;
     p.x_has_lo = x.dtype == CSDR_DTYPE_F32 ? 1u : 0u;
-    p.tmem_cols = std::max(32u, 2u * p.n_tile);
+    p.x_vec = x.layout == CSDR_LAYOUT_TOKEN_MAJOR && x.C % 8u == 0 && (reinterpret_cast<uintptr_t>(x.x) & 15u) == 0;
+    p.tmem_cols = 32u;
+    while (p.tmem_cols < 2u * p.n_tile) p.tmem_cols <<= 1;
     const size_t x_bytes = static_cast<size_t>(p.n_kb) * (p.x_has_lo ? 2u : 1u) * p.n_tile * 128u;
     const size_t smem_max = ctx->smem_optin - 2048u;
+    const uint32_t tok_tiles = (p.n_tok + p.n_tile - 1u) / p.n_tile, tiles = p.rows / kTileM;
+    const uint32_t ctas = std::min(tiles, std::max(1u, static_cast<uint32_t>(ctx->sm_count) / tok_tiles));
     p.stages = static_cast<uint32_t>(std::min<size_t>(kTileStages, (smem_max - 1024u - x_bytes) / (2u * kATile)));
     const size_t smem = x_bytes + static_cast<size_t>(p.stages) * 2u * kATile + 1024u;
     p.status = ctx->status_word;
     p.spin = ctx->spin_limit_barrier;
     ctx->opt_in_smem(reinterpret_cast<const void*>(hsdr_tile_project_mma_kernel), smem);
-    const uint32_t tok_tiles = (p.n_tok + p.n_tile - 1u) / p.n_tile, tiles = p.rows / kTileM;
-    const uint32_t per = std::max(1u, static_cast<uint32_t>(ctx->sm_count) / tok_tiles);
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(std::min(tiles, per), tok_tiles, 1);
+    cfg.gridDim = dim3(ctas, tok_tiles, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;

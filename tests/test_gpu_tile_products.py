@@ -39,6 +39,8 @@ def product(ctx, pay, x, dtype, token, shift=0):
     (256, 512, 128, 128, 160, 8, 2),      # more row tiles than SMs: both accumulators in turn
     (128, 408, 128, 136, 20, 8, 3),       # three column blocks, the last one partly outside
     (256, 512, 32, 32, 16, 4, 15),        # 240 tokens: two token tiles, the second partly outside
+    (128, 384, 128, 128, 160, 8, 13),     # 39 tokens in a tile of 48
+    (128, 576, 32, 32, 20, 4, 8),         # 144 tokens in two tiles of 80
 ])
 def test_tile_products(ctx, oracle, rows, cols, tr, tc, atoms, k, m, dtype, token):
     pay = synth.hsdr_payload(rows, cols, tile_rows=tr, tile_cols=tc, n_atoms=atoms, k=k, seed=rows + tc)
