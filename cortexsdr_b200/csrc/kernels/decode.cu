@@ -87,9 +87,9 @@ hsdr_decode_rows_kernel(const float* __restrict__ D, const uint16_t* __restrict_
 // elements each, so an atom row is one conflict-free 128-bit read per lane. hsdr_decode_rows_kernel
 // re-reads every atom from L2 for every tile instead: 1.6 GB for 4099 x 4101 in 128 x 128 tiles,
 // scalar where the width is odd (365 us); here the same bytes come from shared memory, whose
-// bandwidth (about 45 us of it) and the issue of ten instructions a code are the bound: 75 us, and
-// 65 us where the width is a multiple of four. 32 warps on an SM hide the reads of codes and atoms
-// (16: 86 us). The (slice, tile) pairs are dealt to the CTAs, one an SM, in equal contiguous runs,
+// bandwidth (about 45 us of it) and the issue of ten instructions a code are the bound: 79 us.
+// 32 warps on an SM hide the reads of codes and atoms
+// (16 warps cost 11 us more). The (slice, tile) pairs are dealt to the CTAs, one an SM, in equal contiguous runs,
 // so a CTA stages one to three slices. Sums as above: stage-major, slot-minor, one multiplication and
 // one addition per code, never contracted.
 constexpr uint32_t kTilesThreads = 1024;

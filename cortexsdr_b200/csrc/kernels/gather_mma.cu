@@ -11,8 +11,8 @@
 //     for all three; their sums meet in the epilogue in fp32.
 // hsdr_gather_wide_kernel looks every code up in shared memory instead: S * k * 4 bytes per result,
 // 15 us of shared-memory bandwidth for 11008 rows at 512 tokens behind 2.5 us of staging, 28 us
-// measured; the products here are 10 us of tensor time behind 3.5 us of planes, 19 us measured (the
-// hand-over of a coefficient block to the products, 200 cycles of barrier, is what keeps them waiting).
+// measured; the products here are 10 us of tensor time behind 3.5 us of planes, 19 us measured (what keeps
+// them waiting is the hand-over of coefficient blocks, a barrier each way).
 //
 // Warp 0 fetches the planes by TMA (one barrier per 64 atoms), warp 1 issues the products, warps 2-5 and
 // 6-9 write the even and the odd coefficient blocks into their one of two buffers (a block takes four

@@ -120,7 +120,7 @@ __device__ __forceinline__ void stage_x(const XView& xv, uint32_t c0, uint32_t c
 //   xs      [MT][xcols]    activations (xcols = C when they fit, else one column slab)
 //   codes   per segment: the CTA's rows of the code stream, 16-byte units
 //   scales  per segment: S floats (padded to 4)
-//   dxs     [K][MTG]       Dx slices: of one segment at a time, or of every segment side by side (TOGETHER)
+//   dxs     [K][MTG]       Dx slices: of one segment at a time, or of every segment side by side (Walk::kTogether)
 struct SmemPlan {
     uint32_t xcols;                       // C (whole x resident) or slab
     uint32_t codes_off[kMaxFusedGroup];   // byte offsets

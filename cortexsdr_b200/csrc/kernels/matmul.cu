@@ -9,7 +9,8 @@
 //   hsdr_tile_project/_tile_gather/_edge kernels
 //                           decompress (:1340-1440) followed by the dense product of
 //                           SDRInferenceEngine::matmulForLayer (SparseInferenceEngine.cpp:1301-1310),
-//                           computed in factored form so the weight never exists in memory
+//                           computed in factored form, for the products whose weight is not kept rebuilt
+//                           (launch_matmul says which)
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 

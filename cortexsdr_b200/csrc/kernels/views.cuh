@@ -25,7 +25,7 @@ struct XView {
     uint32_t C;      // features
     uint32_t Mtotal; // tokens in the whole activation matrix
     uint32_t b0;     // first token of this launch's chunk
-    uint32_t M;      // tokens in this chunk (<= MT)
+    uint32_t M;      // tokens in this chunk (<= MT where a kernel has a token tile of its own)
 };
 
 __device__ __forceinline__ float load_x(const XView& v, uint32_t c, uint32_t b) {

@@ -175,7 +175,8 @@ CSDR_API int csdr_unpack_codes(csdr_context* ctx, const csdr_segment* seg, int32
  * and ::matmulWithExternalDictionary (:1830): host buffers, reference layout
  * (x: C x batch, y: R x batch, fp32). As the reference, refuses 2-D tiles
  * (CSDR_ERR_GEOMETRY) unless allow_2d != 0, in which case the result equals the
- * reference's decompress() + dense product (SparseInferenceEngine.cpp:1301-1310). */
+ * reference's decompress() + dense product (SparseInferenceEngine.cpp:1301-1310). A 2-D segment
+ * may keep its weight rebuilt (4 bytes an element) from its first product on, at any batch. */
 CSDR_API int csdr_matmul(csdr_context* ctx, const csdr_segment* seg, const float* x,
                          size_t batch, float* y, int allow_2d);
 /* Same product with device-resident activations. x_dtype/x_layout/y_layout as the
@@ -188,8 +189,9 @@ CSDR_API int csdr_matmul_device_async(csdr_context* ctx, const csdr_segment* seg
                                       const float* bias_dev);
 
 /* Several compressed weights that consume the SAME activations (q|k|v, gate|up) in as few
- * launches as possible: 1-D row-tile segments of equal column count share one kernel,
- * anything else is issued segment by segment. ys_dev[i] receives segment i's product.
+ * launches as possible: 1-D row-tile segments share their projection, and up to sixteen
+ * tokens their gather; 2-D tiles are issued segment by segment. ys_dev[i] receives segment i's
+ * product.
  * The reference issues these as separate matmulHSDR calls
  * (api/cortex_sdk.cpp:1578-1583, :1653-1656). */
 CSDR_API int csdr_matmul_group_device_async(csdr_context* ctx, const csdr_segment* const* segs,
@@ -201,8 +203,9 @@ CSDR_API int csdr_matmul_group_device_async(csdr_context* ctx, const csdr_segmen
  * and gate|up of a block, the experts of a routed layer, a chain of layers. Lists whose members
  * are all 1-D row-tile segments with one common batch of 1 to 4 tokens run as one persistent
  * kernel per 32 tasks, in which the weight stream of task n+1 flows under the hand-over and
- * gather of task n (tasks may differ in shape, activations and outputs); any other list is
- * issued task by task, in order. A task whose activations are another task's output names that
+ * gather of task n (tasks may differ in shape, activations and outputs); any other list gives
+ * what its tasks give one after the other, in order (neighbours that do not touch each other's
+ * operands or results may share launches). A task whose activations are another task's output names that
  * task in after_task (an index below its own, in the same group of 32; -1: none): its weights
  * still stream ahead, its activations are read once that task's rows are complete. The
  * reference issues one matmulHSDR call per product (SparseInferenceEngine.cpp:1074-1091). */
