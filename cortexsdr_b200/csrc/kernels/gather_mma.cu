@@ -179,20 +179,24 @@ struct GatherMmaParams {
     uint32_t spin;
 };
 
-// One result from the row's codes. Rare: a sum that is not finite.
-__device__ __noinline__ float looked_up(const GatherMmaParams& p, uint32_t row, uint32_t tok) {
+// What is not finite among a row's results for n tokens, from the row's codes. Out of the way of the loop
+// that leads here.
+__device__ __noinline__ void look_up(const GatherMmaParams& p, uint32_t row, uint32_t tok, uint32_t n, float* sum) {
     const size_t plane = static_cast<size_t>(p.n_blocks) * kAtomBlock * p.stride;
     const uint16_t* c = p.codes + static_cast<size_t>(row) * p.S * p.k;
-    float sum = 0.0f;
-    for (uint32_t s = 0; s < p.S * p.k; ++s) {
-        const uint32_t code = c[s];
-        const float gamma = p.scales[s / p.k];
-        const __nv_bfloat16* at = p.planes + static_cast<size_t>(code & 0x7FFFu) * p.stride + tok;
-        float v = __bfloat162float(at[0]);
-        if (isfinite(v)) v += __bfloat162float(at[plane]) + __bfloat162float(at[2u * plane]);
-        sum += __fmul_rn((code & 0x8000u) ? -gamma : gamma, v);
+    for (uint32_t j = 0; j < n; ++j) {
+        if (isfinite(sum[j])) continue;
+        float v = 0.0f;
+        for (uint32_t s = 0; s < p.S * p.k; ++s) {
+            const uint32_t code = c[s];
+            const float gamma = p.scales[s / p.k];
+            const __nv_bfloat16* at = p.planes + static_cast<size_t>(code & 0x7FFFu) * p.stride + tok + j;
+            float dx = __bfloat162float(at[0]);
+            if (isfinite(dx)) dx += __bfloat162float(at[plane]) + __bfloat162float(at[2u * plane]);
+            v += __fmul_rn((code & 0x8000u) ? -gamma : gamma, dx);
+        }
+        sum[j] = v;
     }
-    return sum;
 }
 
 // grid (per_slice CTAs over the row tiles, 64-token slices)
@@ -358,6 +362,7 @@ hsdr_gather_mma_kernel(const __grid_constant__ CUtensorMap map, const __grid_con
         const uint32_t tw = min(kTok, p.M - t0) > first ? min(32u, min(kTok, p.M - t0) - first) : 0u;   // this warp's tokens
         const bool feature = p.y.layout == CSDR_LAYOUT_FEATURE_MAJOR;
         const size_t row_step = feature ? p.y.Mtotal : 1u, tok_step = feature ? 1u : p.y.R;
+        uint32_t odd = 0;            // of the warp's two runs of sixteen tokens: some projection is not finite
         for (uint32_t ti = 0; ti < hi - lo; ++ti) {
             const uint32_t acc = ti & 1u;
             if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&acc_full[acc]), (ti / 2u) & 1u, p.spin, failed))) {
@@ -405,19 +410,33 @@ hsdr_gather_mma_kernel(const __grid_constant__ CUtensorMap map, const __grid_con
                     for (uint32_t j = 0; j < 16u; ++j) h[j] = 0.0f;
                 }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                float sum[16], odd = 0.0f;
+                if (ti == 0u) {
+                    // a projection that is not finite leaves NaN in its low plane, so in every row: the first
+                    // tile tells for all
+                    float all[8];
 #pragma unroll
-                for (uint32_t j = 0; j < 16u; ++j) {
-                    sum[j] = __uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j]));
-                    odd = fmaf(sum[j], 0.0f, odd);          // NaN where a sum is not finite
+                    for (uint32_t j = 0; j < 8u; ++j) all[j] = __uint_as_float(r[2][j]) + __uint_as_float(r[2][j + 8u]);
+#pragma unroll
+                    for (uint32_t w = 4u; w > 0u; w >>= 1)
+#pragma unroll
+                        for (uint32_t j = 0; j < w; ++j) all[j] += all[j + w];
+                    if (__any_sync(0xFFFFFFFFu, !isfinite(all[0]))) odd |= 1u << ch;
                 }
-                if (odd != 0.0f) {
+                if (odd >> ch & 1u) {
+                    float again[16];
 #pragma unroll
                     for (uint32_t j = 0; j < 16u; ++j)
-                        if (j < n && !isfinite(sum[j])) sum[j] = looked_up(p, row, t0 + first + ch * 16u + j);
+                        again[j] = __uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j]));
+                    look_up(p, row, t0 + first + ch * 16u, n, again);
+#pragma unroll
+                    for (uint32_t j = 0; j < 16u; ++j) {
+                        r[0][j] = __float_as_uint(again[j]);
+                        r[1][j] = r[2][j] = 0u;
+                    }
                 }
 #pragma unroll
-                for (uint32_t j = 0; j < 16u; ++j) h[j] += fmaf(sum[j], inv_s[first + ch * 16u + j], bias);
+                for (uint32_t j = 0; j < 16u; ++j)
+                    h[j] += fmaf(__uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j])), inv_s[first + ch * 16u + j], bias);
                 if (quads) {
 #pragma unroll
                     for (uint32_t j = 0; j < 16u; j += 4u) *reinterpret_cast<float4*>(dst + j) = make_float4(h[j], h[j + 1], h[j + 2], h[j + 3]);
